@@ -60,14 +60,15 @@ struct RasterArgs {
   int4* bbox;  // {left, right, bottom, top}; empty when culled
   int32_t* tile_count;  // triangles inside one tile (their slots come from here)
   int32_t* tile_multi;  // triangles spanning 2..large_tiles tiles
-  int32_t* tile_fill;   // bin slots taken by the multi-tile triangles; after
-                        // binning, the tiles in the fine rasterizer's order
+  int32_t* tile_fill;   // bin slots taken by the multi-tile triangles
+  uint32_t* order;      // [tiles][3] the fine rasterizer's queue (see pack_tile),
+                        // over the three arrays above once the bins are filled
   int32_t* tile_first;  // exclusive scan of tile_count + tile_multi, total_tiles + 1
   int32_t* bins;        // global triangle indices grouped by tile
   int32_t* large_count;  // per image
   int32_t* large_list;   // per image, at tri_start[image]
-  uint32_t* counters;    // [0] work queue head, [1] error flags, [2, 8) tiles
-                         // per cost class, [8, 14) their fill counts
+  uint32_t* counters;    // [0] work queue head, [1] error flags, [2, 9) tiles
+                         // per cost class, [9, 16) their fill counts
   int32_t* ids;
   float* z;
   float* bary;
@@ -76,7 +77,7 @@ struct RasterArgs {
 
 // Workspace: the zeroed block first, then the rest; 256-byte aligned parts.
 struct Layout {
-  size_t counters, tile_count, tile_multi, tile_fill, large_count, zero_end;
+  size_t counters, tile_count, tile_multi, tile_fill, large_count, zero_end;  // order: tile_count
   size_t tile_first, setup, bbox, bins, large_list, total;
 };
 
@@ -295,14 +296,15 @@ __global__ void __launch_bounds__(256) bin_scatter_kernel(RasterArgs a, Batch B)
 // no block is left with a heavy tile while the others have run out of work
 // (the per-tile cost spans three orders of magnitude in ragged batches). The
 // cost of a tile is its triangle count (binned plus the image's large ones),
-// in six classes, heaviest first; inside a class tiles keep roughly their
-// index order (block by block), which keeps an image's tiles together in L2.
-// The order does not change any output: tiles are independent.
-constexpr int kCostClasses = 6;
+// in seven classes, heaviest first and the empty ones last; inside a class
+// tiles keep roughly their index order (block by block), which keeps an
+// image's tiles together in L2. The order does not change any output: tiles
+// are independent.
+constexpr int kCostClasses = 7, kEmptyClass = kCostClasses - 1;
 
 __device__ __forceinline__ int cost_class(const RasterArgs& a, int tile, int img) {
   const int c = a.tile_first[tile + 1] - a.tile_first[tile] + a.large_count[img];
-  return c >= 512 ? 0 : c >= 128 ? 1 : c >= 32 ? 2 : c >= 8 ? 3 : c >= 2 ? 4 : 5;
+  return c >= 512 ? 0 : c >= 128 ? 1 : c >= 32 ? 2 : c >= 8 ? 3 : c >= 2 ? 4 : c >= 1 ? 5 : 6;
 }
 
 // Tiles per cost class (counters[2 + class]), one shared-memory histogram
@@ -318,17 +320,33 @@ __global__ void __launch_bounds__(256) tile_cost_kernel(RasterArgs a, Batch B) {
     atomicAdd(&a.counters[2 + threadIdx.x], unsigned(h[threadIdx.x]));
 }
 
-// Writes every tile index to its place in the order (tile_fill, free once
-// the bins are filled): class c starts after the tiles of classes < c, and
-// each block takes a run of its classes' slots (counters[8 + class]).
+// A tile of the queue in three words: its first bin slot; its triangles in
+// the bins (27 bits, saturated) and 5 bits of its image; its origin (15 bits
+// each) and 2 more bits of the image (DR_MAX_BATCH_INLINE = 128). One load
+// then tells a block all about its next tile, where looking the image up and
+// reading the bin bounds was a chain of two more loads and two divisions.
+constexpr uint32_t kMaxPackedCount = (1u << 27) - 1;
+static_assert(DR_MAX_BATCH_INLINE <= 128 && DR_MAX_IMAGE_DIM <= 32768, "pack_tile's fields");
+
+__device__ __forceinline__ void pack_tile(uint32_t* o, uint32_t bin0, uint32_t nbin, int img,
+                                          int x0, int y0) {
+  o[0] = bin0;
+  o[1] = min(nbin, kMaxPackedCount) | uint32_t(img & 31) << 27;
+  o[2] = uint32_t(x0) | uint32_t(y0) << 15 | uint32_t(img >> 5) << 30;
+}
+
+// Writes every tile to its place in the order: class c starts after the
+// tiles of classes < c, and each block takes a run of its classes' slots
+// (counters[9 + class]).
 __global__ void __launch_bounds__(256) tile_order_kernel(RasterArgs a, Batch B) {
   __shared__ int h[kCostClasses], base[kCostClasses];
   if (threadIdx.x < kCostClasses) h[threadIdx.x] = 0;
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int c = 0, rank = 0;
+  int c = 0, rank = 0, img = 0;
   if (i < a.total_tiles) {
-    c = cost_class(a, i, find_segment(B.tile_start, B.n, i));
+    img = find_segment(B.tile_start, B.n, i);
+    c = cost_class(a, i, img);
     rank = atomicAdd(&h[c], 1);
   }
   __syncthreads();
@@ -336,10 +354,17 @@ __global__ void __launch_bounds__(256) tile_order_kernel(RasterArgs a, Batch B) 
     int start = 0;
     for (int k = 0; k < int(threadIdx.x); ++k) start += int(a.counters[2 + k]);
     const int n = h[threadIdx.x];
-    base[threadIdx.x] = start + (n ? int(atomicAdd(&a.counters[8 + threadIdx.x], unsigned(n))) : 0);
+    base[threadIdx.x] =
+        start + (n ? int(atomicAdd(&a.counters[2 + kCostClasses + threadIdx.x], unsigned(n))) : 0);
   }
   __syncthreads();
-  if (i < a.total_tiles) a.tile_fill[base[c] + rank] = i;
+  if (i < a.total_tiles) {
+    const int local = i - B.tile_start[img], ntx = B.tiles_x[img];
+    const int ty = local / ntx, tx = local - ty * ntx;
+    const int first = a.tile_first[i];
+    pack_tile(a.order + 3 * size_t(base[c] + rank), first, a.tile_first[i + 1] - first, img,
+              tx * a.TW, ty * a.TH);
+  }
 }
 
 // Per chunk of up to kThreads triangles overlapping the tile, compacted to
@@ -377,67 +402,183 @@ __host__ __device__ inline size_t fine_smem_bytes(int L, int TW, int TH) {
 // (triangle, pixel) candidates of each chunk of the tile's triangles evenly
 // over its threads (block prefix scan + binary search), so large and small
 // triangles cost the same per pixel.
-// Fused interpolation of one layer sample o with triangle `id` and the
-// barycentrics just written: the splat position of a foreground sample
-// (splat.py:207-221) with its clip w, its three vertex indices when
-// requested (the Framebuffer's vertex_ids, rasterize.py:111-113), and the
-// attributes (interpolate.py:24-63, background 0). The same operations, in
-// the same order, as samples_fwd_kernel on the stored buffers.
+// Fused interpolation of one occupied layer sample o, the record of its
+// triangle and the barycentrics just written: the splat position of a
+// foreground sample (splat.py:207-221) with its clip w, its three vertex
+// indices when requested (the Framebuffer's vertex_ids,
+// rasterize.py:111-113), and the attributes (interpolate.py:24-63). The same
+// operations, in the same order, as samples_fwd_kernel on the stored buffers.
+// A depth of exactly 1 is background: its attributes stay as
+// fill_background left them.
 __device__ __forceinline__ void write_sample(const RasterArgs& a, const Batch& B, int img,
                                           const TriSetup* t, float zz, const float b[3],
                                           int64_t o) {
   const SampleOutputs& so = a.so;
   const int K = so.K;
   const bool vec_rows = (K & 3) == 0;
-  float4 c;
-  float* ao = so.attr ? so.attr_out + o * K : nullptr;
-  const bool fg = zz != 1.0f;
-  if (fg) {
-    // One record holds the vertex indices and clip coordinates (the sample
-    // is foreground, so its key and record exist).
-    const float2 z01 = __ldg(reinterpret_cast<const float2*>(t->vz));
-    const int4 r5 = __ldg(reinterpret_cast<const int4*>(t) + 5);  // vz2, vw0..2
-    const int4 r6 = __ldg(reinterpret_cast<const int4*>(t) + 6);  // vid0..2, vx0
-    const int4 r7 = __ldg(reinterpret_cast<const int4*>(t) + 7);  // vx1, vx2, vy0, vy1
-    const int4 r8 = __ldg(reinterpret_cast<const int4*>(t) + 8);  // vy2
-    const int v0 = r6.x, v1 = r6.y, v2 = r6.z;
-    c = lerp_clip(make_float4(__int_as_float(r6.w), __int_as_float(r7.z), z01.x,
-                              __int_as_float(r5.y)),
-                  make_float4(__int_as_float(r7.x), __int_as_float(r7.w), z01.y,
-                              __int_as_float(r5.z)),
-                  make_float4(__int_as_float(r7.y), __int_as_float(r8.x),
-                              __int_as_float(r5.x), __int_as_float(r5.w)), b);
-    if (ao) {
-      const float* ab = so.attr + B.vertex_offset[img] * K;
-      const float* a0 = ab + int64_t(v0) * K;
-      const float* a1 = ab + int64_t(v1) * K;
-      const float* a2 = ab + int64_t(v2) * K;
-      for (int k = 0; k < K; k += 4) {
-        const int n = min(4, K - k);
-        const float4 x = load_chunk(a0 + k, n, vec_rows), y = load_chunk(a1 + k, n, vec_rows),
-                     w = load_chunk(a2 + k, n, vec_rows);
-        store_chunk(ao + k,
-                    make_float4(lerp3(x.x, y.x, w.x, b), lerp3(x.y, y.y, w.y, b),
-                                lerp3(x.z, y.z, w.z, b), lerp3(x.w, y.w, w.w, b)),
-                    n, vec_rows);
+  if (zz == 1.0f) return;
+  // One record holds the vertex indices and clip coordinates.
+  const float2 z01 = __ldg(reinterpret_cast<const float2*>(t->vz));
+  const int4 r5 = __ldg(reinterpret_cast<const int4*>(t) + 5);  // vz2, vw0..2
+  const int4 r6 = __ldg(reinterpret_cast<const int4*>(t) + 6);  // vid0..2, vx0
+  const int4 r7 = __ldg(reinterpret_cast<const int4*>(t) + 7);  // vx1, vx2, vy0, vy1
+  const int4 r8 = __ldg(reinterpret_cast<const int4*>(t) + 8);  // vy2
+  const int v0 = r6.x, v1 = r6.y, v2 = r6.z;
+  const float4 c = lerp_clip(make_float4(__int_as_float(r6.w), __int_as_float(r7.z), z01.x,
+                                         __int_as_float(r5.y)),
+                             make_float4(__int_as_float(r7.x), __int_as_float(r7.w), z01.y,
+                                         __int_as_float(r5.z)),
+                             make_float4(__int_as_float(r7.y), __int_as_float(r8.x),
+                                         __int_as_float(r5.x), __int_as_float(r5.w)), b);
+  if (so.attr) {
+    float* ao = so.attr_out + o * K;
+    const float* ab = so.attr + B.vertex_offset[img] * K;
+    const float* a0 = ab + int64_t(v0) * K;
+    const float* a1 = ab + int64_t(v1) * K;
+    const float* a2 = ab + int64_t(v2) * K;
+    for (int k = 0; k < K; k += 4) {
+      const int n = min(4, K - k);
+      const float4 x = load_chunk(a0 + k, n, vec_rows), y = load_chunk(a1 + k, n, vec_rows),
+                   w = load_chunk(a2 + k, n, vec_rows);
+      store_chunk(ao + k,
+                  make_float4(lerp3(x.x, y.x, w.x, b), lerp3(x.y, y.y, w.y, b),
+                              lerp3(x.z, y.z, w.z, b), lerp3(x.w, y.w, w.w, b)),
+                  n, vec_rows);
+    }
+  }
+  // w carries the interpolated clip w, which the VJP needs (background
+  // and foreground are told apart by the depth buffer).
+  so.positions[o] = viewport_of(c, __int2float_rn(B.width[img]),
+                                __int2float_rn(B.height[img]), c.w);
+  if (so.vertex_ids) {
+    int32_t* vo = so.vertex_ids + 3 * o;
+    vo[0] = v0;
+    vo[1] = v1;
+    vo[2] = v2;
+  }
+}
+
+// One tile of an image in the packed layered buffers.
+struct TileBox {
+  int64_t base;  // element of layer 0, pixel (0, 0)
+  int64_t hw;    // elements per layer
+  int img, W, x0, y0, tw, th;
+  int bin0, nbin;
+};
+
+// Entry k of the queue, as packed by pack_tile.
+__device__ __forceinline__ uint3 tile_words(const RasterArgs& a, int k) {
+  const uint32_t* o = a.order + 3 * size_t(k);
+  return make_uint3(__ldg(o), __ldg(o + 1), __ldg(o + 2));
+}
+
+__device__ __forceinline__ TileBox tile_box(const RasterArgs& a, const Batch& B, uint3 o, int L) {
+  TileBox t;
+  t.img = int((o.y >> 27) | (o.z >> 30) << 5);
+  t.W = B.width[t.img];
+  t.hw = int64_t(t.W) * B.height[t.img];
+  t.base = int64_t(L) * B.pix_off[t.img];
+  t.x0 = int(o.z & 0x7fffu);
+  t.y0 = int((o.z >> 15) & 0x7fffu);
+  t.tw = min(a.TW, t.W - t.x0);
+  t.th = min(a.TH, B.height[t.img] - t.y0);
+  t.bin0 = int(o.x);
+  t.nbin = int(o.y & kMaxPackedCount);
+  if (uint32_t(t.nbin) == kMaxPackedCount) {
+    const int item = B.tile_start[t.img] + (t.y0 / a.TH) * B.tiles_x[t.img] + t.x0 / a.TW;
+    t.nbin = a.tile_first[item + 1] - t.bin0;
+  }
+  return t;
+}
+
+// The fine rasterizer's queue: the occupied tiles in order, then the empty
+// ones kEmptyRun at a time (they only write background samples).
+constexpr int kEmptyRun = 8;
+
+struct Queue {
+  unsigned occupied, items;
+};
+
+__device__ __forceinline__ Queue make_queue(const RasterArgs& a) {
+  const unsigned empty = a.counters[2 + kEmptyClass];
+  Queue q;
+  q.occupied = unsigned(a.total_tiles) - empty;
+  q.items = q.occupied + (empty + kEmptyRun - 1) / kEmptyRun;
+  return q;
+}
+
+// One item as its block sees it.
+struct QueueItem {
+  int kind;  // 0 tile, 1 empty run, 2 end
+  uint3 o;   // tile: its words; run: o.x = its first entry
+};
+
+__device__ __forceinline__ QueueItem queue_item(const RasterArgs& a, const Queue& q,
+                                                unsigned head) {
+  QueueItem it;
+  it.kind = head < q.occupied ? 0 : head < q.items ? 1 : 2;
+  it.o = make_uint3(q.occupied + (head - q.occupied) * kEmptyRun, 0u, 0u);
+  if (it.kind == 0) it.o = tile_words(a, int(head));
+  return it;
+}
+
+// Writes v to the `ch` values of every layer sample of a tile, row by row:
+// consecutive threads take consecutive float4s (floats where a row does not
+// start and end on 16 bytes).
+__device__ __forceinline__ void fill_rows(float* buf, int ch, float v, const TileBox& t, int L) {
+  const int64_t first = (t.base + int64_t(t.y0) * t.W + t.x0) * ch;
+  const int64_t layer = t.hw * ch;
+  const int row = t.W * ch, n = t.tw * ch;
+  const bool vec = (((row | n | int(first) | int(layer)) & 3) |
+                    int(reinterpret_cast<uintptr_t>(buf) & 15)) == 0;
+  const int cols = vec ? n >> 2 : n, step = vec ? 4 : 1;
+  int y0, dy, dc = 0;
+  if ((cols & (cols - 1)) == 0 && cols <= kThreads) {  // whole rows per step, no division
+    const int lg = __ffs(cols) - 1;
+    y0 = threadIdx.x >> lg;
+    dy = kThreads >> lg;
+  } else {
+    y0 = threadIdx.x / cols;
+    dy = kThreads / cols;
+    dc = kThreads - dy * cols;
+  }
+  const int c0 = threadIdx.x - y0 * cols;
+  float* p = buf + first;
+  for (int l = 0; l < L; ++l, p += layer) {
+    int c = c0;
+    for (int y = y0; y < t.th; y += dy) {
+      float* q = p + (y * row + step * c);
+      if (vec)
+        *reinterpret_cast<float4*>(q) = make_float4(v, v, v, v);
+      else
+        *q = v;
+      c += dc;
+      if (c >= cols) {
+        c -= cols;
+        ++y;
       }
     }
-    // w carries the interpolated clip w, which the VJP needs (background
-    // and foreground are told apart by the depth buffer).
-    so.positions[o] = viewport_of(c, __int2float_rn(B.width[img]),
-                                  __int2float_rn(B.height[img]), c.w);
-    if (so.vertex_ids) {
-      int32_t* vo = so.vertex_ids + 3 * o;
-      vo[0] = v0;
-      vo[1] = v1;
-      vo[2] = v2;
-    }
-  } else if (ao && !a.fg_attr) {
-    // Background: attributes 0; the position is left unwritten (consumers
-    // take background samples from the depth buffer).
-    for (int k = 0; k < K; k += 4)
-      store_chunk(ao + k, make_float4(0.0f, 0.0f, 0.0f, 0.0f), min(4, K - k), vec_rows);
   }
+}
+
+// Every sample of a tile as background: depth 1, and the ids, barycentrics
+// and attributes that the flags ask for (positions are left unwritten:
+// consumers take background samples from the depth buffer). Tiles without
+// triangles end here; in the others the occupied samples are overwritten
+// after a block barrier. Whole rows of float4s instead of a test and a store
+// per sample: with it and the packed queue the kernel takes 1029 us instead
+// of 1128 on the 64-mesh ragged batch (28.4 Mpixel, 78% background), 652
+// instead of 737 on the 4 x 2048^2 terrain; the fill itself is bound by HBM
+// (1.7 GB in 0.2 ms of it on the ragged batch).
+template <bool kFused>
+__device__ __forceinline__ void fill_background(const RasterArgs& a, const TileBox& t, int L) {
+  fill_rows(a.z, 1, 1.0f, t, L);
+  if (!a.fg_only) {
+    fill_rows(reinterpret_cast<float*>(a.ids), 1,
+              __int_as_float(a.depth_mode == DR_DEPTH_DISCRETIZED ? 0 : -1), t, L);
+    fill_rows(a.bary, 3, 0.0f, t, L);
+  }
+  if (kFused && a.so.attr && !a.fg_attr) fill_rows(a.so.attr_out, a.so.K, 0.0f, t, L);
 }
 
 // kFused adds the sample outputs to the epilogue. LT > 0 fixes the layer
@@ -447,7 +588,7 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
                                                                              Batch B) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_warp[kThreads / 32];
-  __shared__ int s_item;
+  __shared__ QueueItem s_item;
   __shared__ int s_nfg;
   const int TW = a.TW, TH = a.TH, TP = TW * TH, L = LT > 0 ? LT : a.L;
   FineSmem s;
@@ -468,26 +609,30 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
   const unsigned long long kEmpty = empty_key(a.depth_mode);
   const bool disc = a.depth_mode == DR_DEPTH_DISCRETIZED;
 
+  const Queue queue = make_queue(a);
   for (;;) {
-    if (threadIdx.x == 0) s_item = int(atomicAdd(&a.counters[0], 1u));
+    if (threadIdx.x == 0) s_item = queue_item(a, queue, atomicAdd(&a.counters[0], 1u));
     __syncthreads();
-    if (s_item >= a.total_tiles) break;
-    const int item = a.tile_fill[s_item];  // heaviest tiles first
-    const int img = find_segment(B.tile_start, B.n, item);
-    const int local = item - B.tile_start[img];
-    const int W = B.width[img], H = B.height[img];
-    const int ntx = B.tiles_x[img];
-    const int x0 = (local % ntx) * TW, y0 = (local / ntx) * TH;
-    const int tw = min(TW, W - x0), th = min(TH, H - y0);
+    const QueueItem it = s_item;
+    if (it.kind == 2) break;
+    if (it.kind == 1) {
+      for (int k = int(it.o.x); k < min(int(it.o.x) + kEmptyRun, a.total_tiles); ++k)
+        fill_background<kFused>(a, tile_box(a, B, tile_words(a, k), L), L);
+      __syncthreads();
+      continue;
+    }
+    const TileBox tb = tile_box(a, B, it.o, L);
+    const int img = tb.img;
+    const int W = tb.W, H = B.height[img], x0 = tb.x0, y0 = tb.y0, tw = tb.tw, th = tb.th;
     const int64_t tri0 = B.tri_start[img];
 
+    fill_background<kFused>(a, tb, L);
     for (int p = threadIdx.x; p < L * TP; p += kThreads) s.keys[p] = kEmpty;
     for (int i = threadIdx.x; i < TW + TH; i += kThreads) {
       if (i < TW) s.pxf[i] = pixel_center_fixed(x0 + i, W, disc);
       else s.pyf[i - TW] = pixel_center_fixed(y0 + i - TW, H, disc);
     }
-    const int bin0 = a.tile_first[item];
-    const int nbin = a.tile_first[item + 1] - bin0;
+    const int bin0 = tb.bin0, nbin = tb.nbin;
     const int nlarge = a.large_count[img];
     const int nsrc = nbin + nlarge;
     __syncthreads();
@@ -590,136 +735,64 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
       __syncthreads();
     }
 
-    // Epilogue: unpack, recompute barycentrics (and float depth) of the
-    // winning triangle at each pixel, write all L layers; optionally also
-    // each layer sample's splat position and interpolated attributes.
-    const int64_t HW = int64_t(H) * W;
-    const int64_t base = int64_t(L) * B.pix_off[img];
-    if constexpr (LT > 0) {
-      // Pass 1 writes background samples and lists the occupied slots
-      // (layer * TP + pixel, in the chunk arrays' space, dead by now); pass
-      // 2 runs the occupied slots with full warps.
-      unsigned short* list = reinterpret_cast<unsigned short*>(s.m);
-      if (threadIdx.x == 0) s_nfg = 0;
-      __syncthreads();
-      const int lane = threadIdx.x & 31;
-      for (int p0 = 0; p0 < TP; p0 += kThreads) {
-        const int p = p0 + threadIdx.x;
-        const int lx = p % TW, ly = p / TW;
-        const bool valid = p < TP && lx < tw && ly < th;
-        const int64_t pix = int64_t(y0 + ly) * W + (x0 + lx);
+    // Epilogue: list the occupied slots (layer * TP + pixel, in the chunk
+    // arrays' space, dead by now), then with full warps unpack each, recompute
+    // the barycentrics (and float depth) of its triangle and overwrite the
+    // background that fill_background wrote; optionally also each sample's
+    // splat position and interpolated attributes.
+    unsigned short* list = reinterpret_cast<unsigned short*>(s.m);
+    if (threadIdx.x == 0) s_nfg = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int p0 = 0; p0 < TP; p0 += kThreads) {
+      const int p = p0 + threadIdx.x;
 #pragma unroll
-        for (int l = 0; l < LT; ++l) {
-          const unsigned long long key = valid ? s.keys[l * TP + p] : kEmpty;
-          const bool full = valid && key != kEmpty;
-          const unsigned ball = __ballot_sync(0xffffffffu, full);
-          int slot0 = 0;
-          if (lane == 0 && ball) slot0 = atomicAdd(&s_nfg, __popc(ball));
-          slot0 = __shfl_sync(0xffffffffu, slot0, 0);
-          if (full) {
-            list[slot0 + __popc(ball & ((1u << lane) - 1u))] = (unsigned short)(l * TP + p);
-          } else if (valid) {
-            const int64_t o = base + l * HW + pix;
-            const float b0[3] = {0.0f, 0.0f, 0.0f};
-            a.z[o] = 1.0f;
-            if (!a.fg_only) {
-              a.ids[o] = disc ? 0 : -1;
-              float* bo = a.bary + 3 * o;
-              bo[0] = 0.0f;
-              bo[1] = 0.0f;
-              bo[2] = 0.0f;
-            }
-            if (kFused) write_sample(a, B, img, nullptr, 1.0f, b0, o);
-          }
-        }
+      for (int l = 0; l < L; ++l) {
+        const bool full = p < TP && s.keys[l * TP + p] != kEmpty;
+        const unsigned ball = __ballot_sync(0xffffffffu, full);
+        if (!ball) break;  // layers fill front to back
+        int slot0 = 0;
+        if (lane == 0) slot0 = atomicAdd(&s_nfg, __popc(ball));
+        slot0 = __shfl_sync(0xffffffffu, slot0, 0);
+        if (full) list[slot0 + __popc(ball & ((1u << lane) - 1u))] = (unsigned short)(l * TP + p);
       }
-      __syncthreads();
-      const int nfg = s_nfg;
-      for (int f = threadIdx.x; f < nfg; f += kThreads) {
-        const int q = list[f];
-        const int l = q / TP, p = q - l * TP;
-        const int lx = p % TW, ly = p / TW;
-        const int64_t pix = int64_t(y0 + ly) * W + (x0 + lx);
-        const unsigned long long key = s.keys[q];
-        const int64_t o = base + l * HW + pix;
-        float b[3] = {0.0f, 0.0f, 0.0f};
-        const int id = int(uint32_t(key));
-        const TriSetup* st = a.setup + tri0 + id;
-        long long m[9];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) m[k] = __ldg(&st->m[k]);
-        long long e[3];
-        edge_values(m, s.pxf[lx], s.pyf[ly], e);
-        float bb[3];
-        barycentrics_of(e, bb);
-        float zz;
-        if (disc) {
-          zz = undiscretize_z(uint32_t(key >> 32));
-        } else {
-          const float3 vz = make_float3(__ldg(&st->vz[0]), __ldg(&st->vz[1]), __ldg(&st->vz[2]));
-          const float3 vw = make_float3(__ldg(&st->vw[0]), __ldg(&st->vw[1]), __ldg(&st->vw[2]));
-          zz = fragment_z(bb, vz, vw, false);
-        }
-        if (!disc || zz != 1.0f) { b[0] = bb[0]; b[1] = bb[1]; b[2] = bb[2]; }
-        a.ids[o] = id;
-        a.z[o] = zz;
-        float* bo = a.bary + 3 * o;
-        bo[0] = b[0];
-        bo[1] = b[1];
-        bo[2] = b[2];
-        if (kFused) write_sample(a, B, img, st, zz, b, o);
-      }
-      __syncthreads();
-    } else {
-      // Any layer count: one pass, pixel by pixel.
-      for (int p = threadIdx.x; p < TP; p += kThreads) {
-        const int lx = p % TW, ly = p / TW;
-        if (lx >= tw || ly >= th) continue;
-        const int64_t pix = int64_t(y0 + ly) * W + (x0 + lx);
-        for (int l = 0; l < L; ++l) {
-          const unsigned long long key = s.keys[l * TP + p];
-          const int64_t o = base + l * HW + pix;
-          float b[3] = {0.0f, 0.0f, 0.0f};
-          int id;
-          float zz;
-          const TriSetup* st = nullptr;
-          if (key == kEmpty) {
-            id = disc ? 0 : -1;
-            zz = 1.0f;
-          } else {
-            id = int(uint32_t(key));
-            st = a.setup + tri0 + id;
-            long long m[9];
-  #pragma unroll
-            for (int q = 0; q < 9; ++q) m[q] = __ldg(&st->m[q]);
-            long long e[3];
-            edge_values(m, s.pxf[lx], s.pyf[ly], e);
-            float bb[3];
-            barycentrics_of(e, bb);
-            if (disc) {
-              zz = undiscretize_z(uint32_t(key >> 32));
-            } else {
-              const float3 vz =
-                  make_float3(__ldg(&st->vz[0]), __ldg(&st->vz[1]), __ldg(&st->vz[2]));
-              const float3 vw =
-                  make_float3(__ldg(&st->vw[0]), __ldg(&st->vw[1]), __ldg(&st->vw[2]));
-              zz = fragment_z(bb, vz, vw, false);
-            }
-            if (!disc || zz != 1.0f) { b[0] = bb[0]; b[1] = bb[1]; b[2] = bb[2]; }
-          }
-          a.z[o] = zz;
-          if (!a.fg_only || key != kEmpty) {
-            a.ids[o] = id;
-            float* bo = a.bary + 3 * o;
-            bo[0] = b[0];
-            bo[1] = b[1];
-            bo[2] = b[2];
-          }
-          if (kFused) write_sample(a, B, img, st, zz, b, o);
-        }
-      }
-      __syncthreads();
     }
+    __syncthreads();
+    const int nfg = s_nfg;
+    for (int f = threadIdx.x; f < nfg; f += kThreads) {
+      const int q = list[f];
+      const int l = q / TP, p = q - l * TP;
+      const int lx = p % TW, ly = p / TW;
+      const unsigned long long key = s.keys[q];
+      const int64_t o = tb.base + l * tb.hw + int64_t(y0 + ly) * W + (x0 + lx);
+      float b[3] = {0.0f, 0.0f, 0.0f};
+      const int id = int(uint32_t(key));
+      const TriSetup* st = a.setup + tri0 + id;
+      long long m[9];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) m[k] = __ldg(&st->m[k]);
+      long long e[3];
+      edge_values(m, s.pxf[lx], s.pyf[ly], e);
+      float bb[3];
+      barycentrics_of(e, bb);
+      float zz;
+      if (disc) {
+        zz = undiscretize_z(uint32_t(key >> 32));
+      } else {
+        const float3 vz = make_float3(__ldg(&st->vz[0]), __ldg(&st->vz[1]), __ldg(&st->vz[2]));
+        const float3 vw = make_float3(__ldg(&st->vw[0]), __ldg(&st->vw[1]), __ldg(&st->vw[2]));
+        zz = fragment_z(bb, vz, vw, false);
+      }
+      if (!disc || zz != 1.0f) { b[0] = bb[0]; b[1] = bb[1]; b[2] = bb[2]; }
+      a.ids[o] = id;
+      a.z[o] = zz;
+      float* bo = a.bary + 3 * o;
+      bo[0] = b[0];
+      bo[1] = b[1];
+      bo[2] = b[2];
+      if (kFused) write_sample(a, B, img, st, zz, b, o);
+    }
+    __syncthreads();
   }
 }
 
@@ -896,6 +969,7 @@ int raster_launch(const float* vertices, const int32_t* triangles,
     a.tile_multi = reinterpret_cast<int32_t*>(ws + lay.tile_multi);
     a.tile_fill = reinterpret_cast<int32_t*>(ws + lay.tile_fill);
     a.tile_first = reinterpret_cast<int32_t*>(ws + lay.tile_first);
+    a.order = reinterpret_cast<uint32_t*>(ws + lay.tile_count);
     a.bins = reinterpret_cast<int32_t*>(ws + lay.bins);
     a.large_count = reinterpret_cast<int32_t*>(ws + lay.large_count);
     a.large_list = reinterpret_cast<int32_t*>(ws + lay.large_list);

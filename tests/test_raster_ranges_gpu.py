@@ -1,0 +1,59 @@
+"""GPU rasterizer against the oracle over the ranges its dispatch rules split:
+edge-function magnitudes, row alignments and channel counts of the background
+rows, layer counts."""
+import numpy as np
+import pytest
+import torch
+
+from diffren_gb300 import _lib, kernels
+from oracle import raster
+from test_raster_gpu import _scene, assert_same, run_abi
+
+pytestmark = pytest.mark.gpu
+
+
+# Scaling a scene's clip coordinates by 2^k leaves its image alone and scales
+# the edge coefficients by 2^2k: they cross 2^43 (from where edge functions may
+# wrap) at k of about 4 to 8, the fixed-point coordinates 2^31 at k = 14, and
+# the products wrap and the conversions saturate above that.
+@pytest.mark.parametrize("kind,n", [("soup", 1500), ("big", 30), ("near", 600)])
+@pytest.mark.parametrize("k", [-9, -4, -1, 0, 1, 2, 3, 4, 6, 9, 13, 14, 15, 18, 23, 31, 48, 60])
+def test_clip_scale_matches_oracle(kind, n, k, device):
+  verts, tris = _scene(kind, n, 96, 71, 3)
+  verts = (np.asarray(verts, np.float64) * 2.0**k).astype(np.float32)
+  for cull, mode, oracle_mode in ((0, _lib.DR_DEPTH_DISCRETIZED, raster.DEPTH_DISCRETIZED),
+                                  (1, _lib.DR_DEPTH_DISCRETIZED, raster.DEPTH_DISCRETIZED),
+                                  (2, _lib.DR_DEPTH_FLOAT, raster.DEPTH_FLOAT)):
+    ref = raster.rasterize(verts, tris, 96, 71, 3, cull, oracle_mode)
+    assert_same(run_abi(verts, tris, 96, 71, 3, cull, mode, device), ref)
+
+
+# Background rows are written as float4s where every row starts and ends on
+# 16 bytes (all of W, tile width and channels decide) and as floats elsewhere;
+# empty tiles go eight at a time; layers are listed up to any L.
+@pytest.mark.parametrize("w,h", [(64, 48), (96, 71), (97, 61), (16, 16), (15, 3), (130, 5), (260, 16)])
+@pytest.mark.parametrize("layers,channels", [(1, 4), (2, 3), (3, 9), (3, 2), (4, 1), (5, 16)])
+def test_background_and_layers_match_oracle(w, h, layers, channels, device):
+  verts, tris = _scene("soup", 60, w, h, 5)
+  clip = torch.tensor(np.asarray(verts, np.float32), device=device)
+  tri = torch.tensor(np.asarray(tris, np.int32), device=device)
+  attr = torch.rand(clip.shape[0], channels, device=device) + 0.5
+  batch = kernels.ImageBatch.single(w, h, clip.shape[0], tri.shape[0])
+  for tile in ((0, 0), (8, 8), (5, 7), (32, 8)):
+    cfg = kernels.raster_config(layers, 1, _lib.DR_DEPTH_DISCRETIZED, tile)
+    ref = raster.rasterize(verts, tris, w, h, layers, 1, raster.DEPTH_DISCRETIZED)
+    n = layers * w * h
+    out = (torch.full((n,), -7, dtype=torch.int32, device=device),
+           torch.full((n,), float("nan"), device=device),
+           torch.full((n, 3), float("nan"), device=device))
+    ids, z, bary = kernels.rasterize_packed(clip, tri, batch, cfg, out=out)
+    assert_same((ids.view(layers, h, w).cpu().numpy(), z.view(layers, h, w).cpu().numpy(),
+                 bary.view(layers, h, w, 3).cpu().numpy()), ref)
+    a, pos, ids2, z2, bary2 = kernels.rasterize_interpolate_packed(
+        attr, clip, tri, batch, cfg, kernels.Workspace(device))
+    assert torch.equal(ids, ids2) and torch.equal(z, z2) and torch.equal(bary, bary2)
+    want, want_pos = kernels.interpolate_with_positions_packed(attr, clip, bary, tri, ids, z,
+                                                               batch, layers)
+    assert torch.equal(a, want)  # 0 on background
+    fg = z != 1.0
+    assert torch.equal(pos[fg][:, :3], want_pos[fg][:, :3])
