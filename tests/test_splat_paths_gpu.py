@@ -1,0 +1,95 @@
+"""The splat forward's and the samples VJP's dispatch edges: pixels whose
+surroundings hold foreground in layer 0 only, sample counts and image sizes on
+both sides of the VJP's block rule."""
+import numpy as np
+import pytest
+import torch
+
+from diffren_gb300 import _lib, kernels, workloads
+
+pytestmark = pytest.mark.gpu
+
+
+# Both calls see the same samples; without a depth buffer the foreground
+# weight travels in the positions and every pixel takes the general surface
+# test, so the images agree bit for bit (also for equal, infinite and NaN
+# depths, whose comparisons are all false).
+@pytest.mark.parametrize("layers", [1, 2, 3, 5, 9])
+@pytest.mark.parametrize("channels", [1, 3, 4, 7])
+def test_single_layer_surroundings_match_general_test(layers, channels, device):
+  w, h = 75, 50
+  g = torch.Generator(device=device).manual_seed(layers * 16 + channels)
+  rand = lambda *s: torch.rand(*s, generator=g, device=device)
+  count = torch.zeros(h, w, dtype=torch.long, device=device)  # foreground layers per pixel
+  count[4:46, 3:70] = 1
+  count[20:30, 40:60] = min(2, layers)
+  count[33:, 10:20] = layers
+  count[rand(h, w) < 0.2] = 0
+  z = torch.full((layers, h, w), 1.0, device=device)
+  depth = 0.5 + 0.49 * rand(layers, h, w)
+  depth = torch.where(rand(layers, h, w) < 0.3, torch.round(depth * 8) / 8 - 0.01, depth)
+  depth[:, 10, 10:14] = float("nan")
+  depth[:, 12, 10:14] = float("inf")
+  fg = torch.arange(layers, device=device)[:, None, None] < count
+  z[fg] = 0.5
+  pos = torch.zeros(layers, h, w, 4, device=device)
+  pos[..., 0] = torch.arange(w, device=device) + 0.5 + 0.2 * (rand(layers, h, w) - 0.5)
+  pos[..., 1] = torch.arange(h, device=device)[:, None] + 0.5 + 0.2 * (rand(layers, h, w) - 0.5)
+  pos[..., 2] = torch.where(fg, depth, torch.ones_like(depth))
+  pos[..., 3] = fg.float()
+  colors = rand(layers, h, w, channels)
+  batch = kernels.ImageBatch.single(w, h, 0, 0)
+  flat = pos.view(-1, 4)
+  general = kernels.splat_packed(flat, colors.view(-1, channels), batch, layers)
+  for grad in (False, True):  # one block per tile, and the listed tiles
+    c = colors.view(-1, channels).clone().requires_grad_(grad)
+    out = kernels.splat_packed(flat, c, batch, layers, z=z.view(-1)).detach()
+    assert torch.equal(out, general) and not torch.isnan(out).any()
+
+
+def _reference(attr, clip, bary, vid, sizes, g_attr, g_pos):
+  """64-bit gradients of the interpolation and the splat positions of
+  foreground samples."""
+  attr = attr.double().requires_grad_()
+  clip = clip.double().requires_grad_()
+  b = bary.double()[:, :, None]
+  a = (attr[vid] * b).sum(1)
+  c = (clip[vid] * b).sum(1)
+  xy = (c[:, :2] / c[:, 3:] + 1.0) * sizes * 0.5
+  loss = (a * g_attr.double()).sum() + (xy * g_pos.double()[:, :2]).sum()
+  return torch.autograd.grad(loss, [attr, clip])
+
+
+# One sample a thread below 3.7 M samples, eight above; a block that spans
+# images looks each sample up.
+@pytest.mark.parametrize("sizes,layers,channels", [
+    ([(9, 7)] * 40, 3, 4), ([(1, 1), (33, 5), (64, 64), (3, 100)], 2, 3), ([(300, 211)], 1, 5),
+    ([(1201, 1050)], 3, 4), ([(640, 480)] * 5 + [(31, 17)] * 30 + [(900, 800)], 2, 2)])
+@pytest.mark.parametrize("deterministic", [False, True])
+def test_samples_vjp_block_rule(sizes, layers, channels, deterministic, device):
+  n = len(sizes)
+  m = workloads.soup_workload(400, seed=3, mu=-2.0, sigma=0.5)
+  eyes = workloads.sphere_eyes(n, seed=4)
+  cams = torch.tensor(np.stack([workloads.camera_matrix(e, w, h)
+                                for e, (w, h) in zip(eyes, sizes)]), device=device)
+  V, T = len(m.vertices), len(m.triangles)
+  batch = kernels.ImageBatch([s[0] for s in sizes], [s[1] for s in sizes], [V] * n, [T] * n)
+  verts = torch.tensor(m.vertices, device=device).repeat(n, 1)
+  tri = torch.tensor(m.triangles, device=device).repeat(n, 1)
+  clip = kernels.transform(verts, cams, batch).requires_grad_()
+  g = torch.Generator(device=device).manual_seed(1)
+  attr = torch.rand(n * V, channels, generator=g, device=device).requires_grad_()
+  cfg = kernels.raster_config(layers, 1, _lib.DR_DEPTH_DISCRETIZED)
+  a, pos, ids, z, bary = kernels.rasterize_interpolate_packed(
+      attr, clip, tri, batch, cfg, kernels.Workspace(device), deterministic=deterministic)
+  g_attr = torch.randn(a.shape, generator=g, device=device)
+  g_pos = torch.randn(pos.shape, generator=g, device=device)
+  got = torch.autograd.grad([a, pos], [attr, clip], [g_attr, g_pos])
+  per = torch.tensor([layers * w * h for w, h in sizes], device=device)
+  img = torch.repeat_interleave(torch.arange(n, device=device), per)
+  fg = z != 1.0
+  vid = tri[img[fg] * T + ids[fg].long()].long() + V * img[fg][:, None]
+  wh = torch.tensor(sizes, dtype=torch.float64, device=device)[img[fg]]
+  want = _reference(attr.detach(), clip.detach(), bary[fg], vid, wh, g_attr[fg], g_pos[fg])
+  for x, y in zip(got, want):
+    assert (x.double() - y).abs().max() <= 1e-4 * y.abs().max()
