@@ -54,21 +54,27 @@ struct RasterArgs {
   int culling, depth_mode, L, TW, TH, large_tiles;
   bool fg_only;  // DR_RASTER_FOREGROUND_ONLY: background ids / barycentrics unwritten
   bool fg_attr;  // DR_RASTER_FOREGROUND_ATTRIBUTES: background attributes unwritten
+  uint32_t inv_tw, inv_th;  // ceil(2^32 / TW), ceil(2^32 / TH) (see tile_index)
   int64_t total_tris;
   int32_t total_tiles;
+  int scan_shift;  // tiles per block of tile_scan_kernel, as a power of two
   TriSetup* setup;
-  int4* bbox;  // {left, right, bottom, top}; empty when culled
+  uint2* box;   // left | right << 16, bottom | top << 16; empty when culled
+  int2* place;  // inside one tile: {tile, slot}; in 2..large_tiles tiles:
+                // {-2, -}; otherwise {-1, -}
   int32_t* tile_count;  // triangles inside one tile (their slots come from here)
   int32_t* tile_multi;  // triangles spanning 2..large_tiles tiles
   int32_t* tile_fill;   // bin slots taken by the multi-tile triangles
   uint32_t* order;      // [tiles][3] the fine rasterizer's queue (see pack_tile),
                         // over the three arrays above once the bins are filled
-  int32_t* tile_first;  // exclusive scan of tile_count + tile_multi, total_tiles + 1
+  int32_t* tile_first;  // first bin of each tile; the tiles of one scan block
+                        // follow each other (see tile_end)
   int32_t* bins;        // global triangle indices grouped by tile
   int32_t* large_count;  // per image
   int32_t* large_list;   // per image, at tri_start[image]
   uint32_t* counters;    // [0] work queue head, [1] error flags, [2, 9) tiles
-                         // per cost class, [9, 16) their fill counts
+                         // per cost class, [9, 16) their fill counts, [16]
+                         // bins taken, [17, 49) end of each scan block's bins
   int32_t* ids;
   float* z;
   float* bary;
@@ -78,7 +84,7 @@ struct RasterArgs {
 // Workspace: the zeroed block first, then the rest; 256-byte aligned parts.
 struct Layout {
   size_t counters, tile_count, tile_multi, tile_fill, large_count, zero_end;  // order: tile_count
-  size_t tile_first, setup, bbox, bins, large_list, total;
+  size_t tile_first, setup, box, place, bins, large_list, total;
 };
 
 size_t align_up(size_t x) { return (x + 255) & ~size_t(255); }
@@ -86,7 +92,7 @@ size_t align_up(size_t x) { return (x + 255) & ~size_t(255); }
 Layout make_layout(int64_t tris, int64_t tiles, int images, int large_tiles) {
   Layout l;
   size_t o = 0;
-  l.counters = o; o = align_up(o + 64);  // queue head, error flags, tile order counts
+  l.counters = o; o = align_up(o + 256);
   l.tile_count = o; o = align_up(o + 4 * tiles);
   l.tile_multi = o; o = align_up(o + 4 * tiles);
   l.tile_fill = o; o = align_up(o + 4 * tiles);
@@ -94,7 +100,7 @@ Layout make_layout(int64_t tris, int64_t tiles, int images, int large_tiles) {
   l.zero_end = o;
   l.tile_first = o; o = align_up(o + 4 * (tiles + 1));
   l.setup = o; o = align_up(o + sizeof(TriSetup) * tris);
-  l.bbox = o; o = align_up(o + 16 * tris);
+  l.box = o; l.place = o + 8 * tris; o = align_up(o + 16 * tris);
   l.bins = o; o = align_up(o + 4 * size_t(large_tiles) * tris);
   l.large_list = o; o = align_up(o + 4 * tris);
   l.total = o;
@@ -123,20 +129,39 @@ __device__ bool cannot_cover(const long long m[9], int4 box, int W, int H, bool 
   return s00 <= 0 && s10 <= 0 && s01 <= 0 && s11 <= 0;
 }
 
-__device__ __forceinline__ void tile_rect(int4 box, int TW, int TH, int& tx0,
-                                          int& tx1, int& ty0, int& ty1) {
-  tx0 = box.x / TW;
-  tx1 = (box.y - 1) / TW;
-  ty0 = box.z / TH;
-  ty1 = (box.w - 1) / TH;
+// x / size for x < 2^16 and size <= 128, by the reciprocal ceil(2^32 / size)
+// (of size 1 it would not fit).
+__device__ __forceinline__ int tile_index(int x, int size, uint32_t inv) {
+  return size == 1 ? x : int(__umulhi(uint32_t(x), inv));
+}
+
+__device__ __forceinline__ void tile_rect(const RasterArgs& a, int4 box, int& tx0, int& tx1,
+                                          int& ty0, int& ty1) {
+  tx0 = tile_index(box.x, a.TW, a.inv_tw);
+  tx1 = tile_index(box.y - 1, a.TW, a.inv_tw);
+  ty0 = tile_index(box.z, a.TH, a.inv_th);
+  ty1 = tile_index(box.w - 1, a.TH, a.inv_th);
+}
+
+// Image sides are at most 32768, so a box's four bounds pack into 16 bits each.
+__device__ __forceinline__ int4 unpack_box(uint2 b) {
+  return make_int4(int(b.x & 0xffffu), int(b.x >> 16), int(b.y & 0xffffu), int(b.y >> 16));
+}
+
+// End of tile i's bins.
+__device__ __forceinline__ int tile_end(const RasterArgs& a, int i) {
+  const int mask = (1 << a.scan_shift) - 1;
+  return (i & mask) == mask || i + 1 == a.total_tiles ? int(a.counters[17 + (i >> a.scan_shift)])
+                                                      : a.tile_first[i + 1];
 }
 
 // One thread per triangle of the batch: bounding box, edge matrix, exact
 // coverage cull, per-tile counts (small triangles) or the large list.
-// Bounded to 64 registers so that four blocks share an SM: the kernel waits
-// on its index and vertex loads, and the extra warps hide more of that than
-// the few bytes of spills cost (measured against three blocks and five).
-__global__ void __launch_bounds__(256, 4) setup_kernel(RasterArgs a, Batch B) {
+// Bounded to 64 registers so that 32 warps share an SM: the kernel waits on
+// its index and vertex loads, and the extra warps hide more of that than the
+// few bytes of spills cost (measured against 24 warps and 40; blocks of 128
+// threads a little faster than of 256).
+__global__ void __launch_bounds__(128, 8) setup_kernel(RasterArgs a, Batch B) {
   const int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   // Lanes past the end still take part in the warp-wide tile match below.
@@ -181,9 +206,9 @@ __global__ void __launch_bounds__(256, 4) setup_kernel(RasterArgs a, Batch B) {
     }
   }
   if (!valid) box = make_int4(0, 0, 0, 0);
-  if (live) a.bbox[g] = box;
+  if (live) a.box[g] = make_uint2(unsigned(box.x | box.y << 16), unsigned(box.z | box.w << 16));
   int tx0 = 0, tx1 = -1, ty0 = 0, ty1 = -1;
-  if (valid) tile_rect(box, a.TW, a.TH, tx0, tx1, ty0, ty1);
+  if (valid) tile_rect(a, box, tx0, tx1, ty0, ty1);
   const int n = (tx1 - tx0 + 1) * (ty1 - ty0 + 1);
   const int base = B.tile_start[img], tx = B.tiles_x[img];
   // Triangles inside one tile count with one atomic per tile per warp.
@@ -191,15 +216,16 @@ __global__ void __launch_bounds__(256, 4) setup_kernel(RasterArgs a, Batch B) {
   const int tile0 = base + ty0 * tx + tx0;
   const unsigned group = __match_any_sync(0xffffffffu, single ? tile0 : -1 - lane);
   if (single) {
-    // The warp's triangles in this tile take consecutive slots; the slot is
-    // kept in the setup record, so the binning pass needs no atomic.
+    // The warp's triangles in this tile take consecutive slots, so that the
+    // binning pass needs no atomic.
     const int leader = __ffs(group) - 1;
     int first = 0;
     if (lane == leader) first = atomicAdd(&a.tile_count[tile0], __popc(group));
     first = __shfl_sync(group, first, leader);
-    a.setup[g].pad[0] = first + __popc(group & ((1u << lane) - 1u));
+    a.place[g] = make_int2(tile0, first + __popc(group & ((1u << lane) - 1u)));
     return;
   }
+  if (live) a.place[g] = make_int2(valid && n <= a.large_tiles ? -2 : -1, 0);
   if (!valid) return;
   if (n <= a.large_tiles) {
     for (int y = ty0; y <= ty1; ++y)
@@ -208,88 +234,6 @@ __global__ void __launch_bounds__(256, 4) setup_kernel(RasterArgs a, Batch B) {
     const int slot = atomicAdd(&a.large_count[img], 1);
     a.large_list[B.tri_start[img] + slot] = int(g);
   }
-}
-
-// Exclusive scan of the per-tile counts (one block; tiles are few). A pass
-// covers 16 Ki counts: warp w owns 512 consecutive counts, read 32 at a time
-// with coalesced loads and scanned with warp shuffles, then the 32 warp
-// totals are scanned once; the next pass's counts load meanwhile.
-__global__ void __launch_bounds__(1024) tile_scan_kernel(const int32_t* count,
-                                                         const int32_t* multi,
-                                                         int32_t* first, int n) {
-  __shared__ int warp_sums[32];
-  constexpr int kRounds = 16, kChunk = 1024 * kRounds;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int carry = 0;
-  int v[kRounds], next[kRounds];
-  const auto load = [&](int base, int (&dst)[kRounds]) {
-#pragma unroll
-    for (int j = 0; j < kRounds; ++j) {
-      const int i = base + warp * (32 * kRounds) + j * 32 + lane;
-      dst[j] = i < n ? __ldg(count + i) + __ldg(multi + i) : 0;
-    }
-  };
-  load(0, v);
-  for (int base = 0; base < n; base += kChunk) {
-    if (base + kChunk < n) load(base + kChunk, next);
-    int run = 0;
-#pragma unroll
-    for (int j = 0; j < kRounds; ++j) {
-      const int inc = warp_inclusive_scan(v[j]);
-      const int excl = run + inc - v[j];
-      run += __shfl_sync(0xffffffffu, inc, 31);
-      v[j] = excl;  // exclusive prefix inside the warp's 512 counts
-    }
-    if (lane == 0) warp_sums[warp] = run;
-    __syncthreads();
-    if (warp == 0) warp_sums[lane] = warp_inclusive_scan(warp_sums[lane]);
-    __syncthreads();
-    const int offset = carry + (warp ? warp_sums[warp - 1] : 0);
-#pragma unroll
-    for (int j = 0; j < kRounds; ++j) {
-      const int i = base + warp * (32 * kRounds) + j * 32 + lane;
-      if (i < n) first[i] = offset + v[j];
-    }
-    carry += warp_sums[31];  // the same in every thread
-    __syncthreads();          // warp_sums is rewritten by the next pass
-#pragma unroll
-    for (int j = 0; j < kRounds; ++j) v[j] = next[j];
-  }
-  if (threadIdx.x == 0) first[n] = carry;
-}
-
-// One thread per triangle: writes its index into the bin of every tile its
-// box touches. Order inside a bin is irrelevant to the result.
-__global__ void __launch_bounds__(256) bin_scatter_kernel(RasterArgs a, Batch B) {
-  const int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  bool binned = false;
-  int tx0 = 0, tx1 = -1, ty0 = 0, ty1 = -1, base = 0, tx = 0;
-  if (g < a.total_tris) {
-    const int4 box = a.bbox[g];
-    if (box.y > box.x) {
-      tile_rect(box, a.TW, a.TH, tx0, tx1, ty0, ty1);
-      if ((tx1 - tx0 + 1) * (ty1 - ty0 + 1) <= a.large_tiles) {
-        binned = true;
-        const int img = find_segment(B.tri_start, B.n, g);
-        base = B.tile_start[img];
-        tx = B.tiles_x[img];
-      }
-    }
-  }
-  // Triangles inside one tile (most of them) took their slot in setup;
-  // the multi-tile ones take theirs after the tile's single-tile triangles.
-  if (!binned) return;
-  if (tx0 == tx1 && ty0 == ty1) {
-    const int tile0 = base + ty0 * tx + tx0;
-    a.bins[a.tile_first[tile0] + a.setup[g].pad[0]] = int(g);
-    return;
-  }
-  for (int y = ty0; y <= ty1; ++y)
-    for (int x = tx0; x <= tx1; ++x) {
-      const int tile = base + y * tx + x;
-      const int pos = a.tile_first[tile] + a.tile_count[tile] + atomicAdd(&a.tile_fill[tile], 1);
-      a.bins[pos] = int(g);
-    }
 }
 
 // Tile order of the fine rasterizer: the most expensive tiles first, so that
@@ -302,22 +246,113 @@ __global__ void __launch_bounds__(256) bin_scatter_kernel(RasterArgs a, Batch B)
 // are independent.
 constexpr int kCostClasses = 7, kEmptyClass = kCostClasses - 1;
 
-__device__ __forceinline__ int cost_class(const RasterArgs& a, int tile, int img) {
-  const int c = a.tile_first[tile + 1] - a.tile_first[tile] + a.large_count[img];
+__device__ __forceinline__ int cost_class(int c) {
   return c >= 512 ? 0 : c >= 128 ? 1 : c >= 32 ? 2 : c >= 8 ? 3 : c >= 2 ? 4 : c >= 1 ? 5 : 6;
 }
 
-// Tiles per cost class (counters[2 + class]), one shared-memory histogram
-// per block.
-__global__ void __launch_bounds__(256) tile_cost_kernel(RasterArgs a, Batch B) {
+// Bins of every tile, and the tiles of each cost class (counters[2 + class]).
+// Blocks take 2^scan_shift tiles each (at most 32 blocks) and their bins from
+// a counter: where a tile's bins lie does not matter, so no block waits for
+// another. One block scanning every count took 30 us for 111k tiles, this 5.
+__global__ void __launch_bounds__(1024) tile_scan_kernel(RasterArgs a, Batch B) {
+  __shared__ int warp_sums[32];
+  __shared__ int s_base;
   __shared__ int h[kCostClasses];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r0 = blockIdx.x << a.scan_shift;
+  const int r1 = min(a.total_tiles, r0 + (1 << a.scan_shift));
+  // Counts past the last tile are zeros (the arrays are padded and cleared).
+  const auto counts = [&](int i) {
+    const int4 c = *reinterpret_cast<const int4*>(a.tile_count + i);
+    const int4 m = *reinterpret_cast<const int4*>(a.tile_multi + i);
+    return make_int4(c.x + m.x, c.y + m.y, c.z + m.z, c.w + m.w);
+  };
   if (threadIdx.x < kCostClasses) h[threadIdx.x] = 0;
+  int sum = 0;
+  for (int i = r0 + 4 * int(threadIdx.x); i < r1; i += 4 * 1024) {
+    const int4 c = counts(i);
+    sum += c.x + c.y + c.z + c.w;
+  }
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if (lane == 0) warp_sums[warp] = sum;
   __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < a.total_tiles) atomicAdd(&h[cost_class(a, i, find_segment(B.tile_start, B.n, i))], 1);
+  if (warp == 0) {
+    sum = __reduce_add_sync(0xffffffffu, warp_sums[lane]);
+    if (lane == 0) {
+      s_base = int(atomicAdd(&a.counters[16], unsigned(sum)));
+      a.counters[17 + blockIdx.x] = unsigned(s_base + sum);
+    }
+  }
+  __syncthreads();
+  int carry = s_base;
+  for (int base = r0; base < r1; base += 4 * 1024) {
+    const int i = base + 4 * int(threadIdx.x);
+    const int4 c = i < r1 ? counts(i) : make_int4(0, 0, 0, 0);
+    const int four = c.x + c.y + c.z + c.w;
+    const int inc = warp_inclusive_scan(four);
+    __syncthreads();  // warp_sums of the pass before has been read
+    if (lane == 31) warp_sums[warp] = inc;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < 32; ++w) {
+      const int v = warp_sums[w];
+      before += w < warp ? v : 0;
+      all += v;
+    }
+    if (i < r1) {
+      const int first = carry + before + inc - four;
+      *reinterpret_cast<int4*>(a.tile_first + i) =
+          make_int4(first, first + c.x, first + c.x + c.y, first + c.x + c.y + c.z);
+      const int n[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (i + k < a.total_tiles)
+          atomicAdd(&h[cost_class(n[k] + a.large_count[find_segment(B.tile_start, B.n, i + k)])], 1);
+    }
+    carry += all;
+  }
   __syncthreads();
   if (threadIdx.x < kCostClasses && h[threadIdx.x])
     atomicAdd(&a.counters[2 + threadIdx.x], unsigned(h[threadIdx.x]));
+}
+
+// One thread per triangle: writes its index into the bin of every tile its
+// box touches. Order inside a bin is irrelevant to the result. Triangles
+// inside one tile (most of them) took their slot in setup; the multi-tile
+// ones take theirs after the tile's single-tile triangles.
+__global__ void __launch_bounds__(256) bin_scatter_kernel(RasterArgs a, Batch B) {
+  const int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (g >= a.total_tris) return;
+  const int2 place = a.place[g];
+  if (place.x >= 0) {
+    a.bins[a.tile_first[place.x] + place.y] = int(g);
+    return;
+  }
+  if (place.x != -2) return;
+  int tx0, tx1, ty0, ty1;
+  tile_rect(a, unpack_box(a.box[g]), tx0, tx1, ty0, ty1);
+  const int img = find_segment(B.tri_start, B.n, g);
+  const int base = B.tile_start[img], ntx = B.tiles_x[img];
+  // Four tiles at a time, so that their atomics' latencies overlap.
+  int x = tx0, y = ty0;
+  while (y <= ty1) {
+    int tile[4], pos[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      tile[k] = y <= ty1 ? base + y * ntx + x : -1;
+      if (++x > tx1) {
+        x = tx0;
+        ++y;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (tile[k] >= 0)
+        pos[k] = a.tile_first[tile[k]] + a.tile_count[tile[k]] + atomicAdd(&a.tile_fill[tile[k]], 1);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (tile[k] >= 0) a.bins[pos[k]] = int(g);
+  }
 }
 
 // A tile of the queue in three words: its first bin slot; its triangles in
@@ -343,10 +378,12 @@ __global__ void __launch_bounds__(256) tile_order_kernel(RasterArgs a, Batch B) 
   if (threadIdx.x < kCostClasses) h[threadIdx.x] = 0;
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int c = 0, rank = 0, img = 0;
+  int c = 0, rank = 0, img = 0, first = 0, n_bin = 0;
   if (i < a.total_tiles) {
     img = find_segment(B.tile_start, B.n, i);
-    c = cost_class(a, i, img);
+    first = a.tile_first[i];
+    n_bin = tile_end(a, i) - first;
+    c = cost_class(n_bin + a.large_count[img]);
     rank = atomicAdd(&h[c], 1);
   }
   __syncthreads();
@@ -361,9 +398,7 @@ __global__ void __launch_bounds__(256) tile_order_kernel(RasterArgs a, Batch B) 
   if (i < a.total_tiles) {
     const int local = i - B.tile_start[img], ntx = B.tiles_x[img];
     const int ty = local / ntx, tx = local - ty * ntx;
-    const int first = a.tile_first[i];
-    pack_tile(a.order + 3 * size_t(base[c] + rank), first, a.tile_first[i + 1] - first, img,
-              tx * a.TW, ty * a.TH);
+    pack_tile(a.order + 3 * size_t(base[c] + rank), first, n_bin, img, tx * a.TW, ty * a.TH);
   }
 }
 
@@ -518,7 +553,7 @@ __device__ __forceinline__ TileBox tile_box(const RasterArgs& a, const Batch& B,
   t.nbin = int(o.y & kMaxPackedCount);
   if (uint32_t(t.nbin) == kMaxPackedCount) {
     const int item = B.tile_start[t.img] + (t.y0 / a.TH) * B.tiles_x[t.img] + t.x0 / a.TW;
-    t.nbin = a.tile_first[item + 1] - t.bin0;
+    t.nbin = tile_end(a, item) - t.bin0;
   }
   return t;
 }
@@ -694,7 +729,7 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
       int cnt = 0, g = 0, cx0 = 0, cy0 = 0, cw = 1;
       if (i < nsrc) {
         g = i < nbin ? a.bins[bin0 + i] : a.large_list[tri0 + (i - nbin)];
-        const int4 box = a.bbox[g];
+        const int4 box = unpack_box(a.box[g]);
         cx0 = max(box.x, x0) - x0;
         cy0 = max(box.z, y0) - y0;
         const int cx1 = min(box.y, x0 + tw) - x0, cy1 = min(box.w, y0 + th) - y0;
@@ -1073,8 +1108,13 @@ int raster_launch(const float* vertices, const int32_t* triangles,
     a.L = L; a.TW = TW; a.TH = TH; a.large_tiles = large;
     a.total_tris = tris;
     a.total_tiles = tiles;
+    a.inv_tw = TW > 1 ? 0xffffffffu / unsigned(TW) + 1u : 0u;
+    a.inv_th = TH > 1 ? 0xffffffffu / unsigned(TH) + 1u : 0u;
+    a.scan_shift = 12;  // 4096 tiles per block, more above 32 blocks
+    while (((int64_t(tiles) + (int64_t(1) << a.scan_shift) - 1) >> a.scan_shift) > 32) ++a.scan_shift;
     a.setup = reinterpret_cast<TriSetup*>(ws + lay.setup);
-    a.bbox = reinterpret_cast<int4*>(ws + lay.bbox);
+    a.box = reinterpret_cast<uint2*>(ws + lay.box);
+    a.place = reinterpret_cast<int2*>(ws + lay.place);
     a.tile_count = reinterpret_cast<int32_t*>(ws + lay.tile_count);
     a.tile_multi = reinterpret_cast<int32_t*>(ws + lay.tile_multi);
     a.tile_fill = reinterpret_cast<int32_t*>(ws + lay.tile_fill);
@@ -1094,17 +1134,19 @@ int raster_launch(const float* vertices, const int32_t* triangles,
       return DR_ERR_CUDA;
     }
     if (tris > 0) {
-      const unsigned grid = unsigned((tris + 255) / 256);
-      setup_kernel<<<grid, 256, 0, stream>>>(a, b);
+      const unsigned grid = unsigned((tris + 127) / 128);
+      setup_kernel<<<grid, 128, 0, stream>>>(a, b);
     }
-    tile_scan_kernel<<<1, 1024, 0, stream>>>(a.tile_count, a.tile_multi, a.tile_first, tiles);
+    if (tiles > 0) {
+      const unsigned grid = unsigned((int64_t(tiles) + (int64_t(1) << a.scan_shift) - 1) >> a.scan_shift);
+      tile_scan_kernel<<<grid, 1024, 0, stream>>>(a, b);
+    }
     if (tris > 0) {
       const unsigned grid = unsigned((tris + 255) / 256);
       bin_scatter_kernel<<<grid, 256, 0, stream>>>(a, b);
     }
     if (tiles > 0) {
       const unsigned grid = unsigned((tiles + 255) / 256);
-      tile_cost_kernel<<<grid, 256, 0, stream>>>(a, b);
       tile_order_kernel<<<grid, 256, 0, stream>>>(a, b);
     }
     const int blocks = std::max(1, std::min(tiles, sms * per_sm));
