@@ -151,13 +151,33 @@ __device__ __forceinline__ long long shl16(long long a) {
   return (long long)((unsigned long long)a << 16);
 }
 
+// __ll2float_rn and __float2ll_rz in 32-bit instructions (the hardware's
+// 64-bit conversions run on the FP64 pipe, of which a GB300 SM has two lanes).
+// float(u), u < 2^46, rounded to nearest: the two 23-bit halves are exact
+// floats (their bits next to the exponent of 2^23, less 2^23), so the one
+// rounding is that of the fused multiply-add.
+__device__ __forceinline__ float ll_to_float_rn(long long v) {
+  const uint64_t u = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
+  if (u >> 46) return __ll2float_rn(v);
+  const float hi = __uint_as_float(0x4b000000u | uint32_t(u >> 23)) - 8388608.0f;
+  const float lo = __uint_as_float(0x4b000000u | (uint32_t(u) & 0x7fffffu)) - 8388608.0f;
+  const float f = __fmaf_rn(hi, 8388608.0f, lo);
+  return v < 0 ? -f : f;
+}
+
+// Truncation with saturation, NaN to INT64_MIN, as cvt.rzi.s64.f32.
+__device__ __forceinline__ long long float_to_ll_rz(float f) {
+  if (fabsf(f) < 2147483648.0f) return (long long)__float2int_rz(f);
+  const uint32_t bits = __float_as_uint(f), exp = (bits >> 23) & 0xffu;
+  if (exp >= 190u)  // |f| >= 2^63, infinite or NaN
+    return (bits >> 31) || f != f ? (long long)(1ull << 63) : (long long)~(1ull << 63);
+  const long long m = (long long)((uint64_t)((bits & 0x7fffffu) | 0x800000u) << (exp - 150u));
+  return bits >> 31 ? -m : m;
+}
+
 // ToFixedPoint (rasterize_utils.h:57-59): 16 fractional bits.
 __device__ __forceinline__ long long to_fixed(float f) {
-  const float s = __fmul_rn(f, 65536.0f);
-  // Below 2^31 the 32-bit conversion truncates to the same value (NaN fails
-  // the test and takes the 64-bit conversion, which maps it to INT64_MIN).
-  if (fabsf(s) < 2147483648.0f) return (long long)__float2int_rz(s);
-  return __float2ll_rz(s);
+  return float_to_ll_rz(__fmul_rn(f, 65536.0f));
 }
 
 // AddPoint (rasterize_utils.h:75-84) on the running box {l, r, b, t}.
@@ -224,31 +244,63 @@ __device__ __forceinline__ bool triangle_box(float4 v0, float4 v1, float4 v2,
   return (r > l) && (t > b);
 }
 
+// Whether the x, y and w of a triangle fit 32 bits in 16.16 fixed point (all
+// but huge coordinates do).
+__device__ __forceinline__ bool fits_fixed32(float4 v0, float4 v1, float4 v2) {
+  // Coordinates below 2^15 (a NaN fails its comparison).
+  const float lim = 32768.0f;
+  return fabsf(v0.x) < lim && fabsf(v0.y) < lim && fabsf(v0.w) < lim && fabsf(v1.x) < lim &&
+         fabsf(v1.y) < lim && fabsf(v1.w) < lim && fabsf(v2.x) < lim && fabsf(v2.y) < lim &&
+         fabsf(v2.w) < lim;
+}
+
 // ComputeUnnormalizedMatrixInverse (rasterize_utils.h:176-206) of the matrix
 // with columns (x_i, y_i, w_i) in 16.16 fixed point. Row i of m holds the
 // coefficients (a, b, c) of edge function i. For NONE and FRONT the reference
 // scales each int64 entry by a float sign, which rounds it to float
 // precision; that rounding is part of the result.
-__device__ __forceinline__ void edge_matrix(float4 v0, float4 v1, float4 v2,
-                                            int culling, long long m[9]) {
-  const long long x0 = to_fixed(v0.x), x1 = to_fixed(v1.x), x2 = to_fixed(v2.x);
-  const long long y0 = to_fixed(v0.y), y1 = to_fixed(v1.y), y2 = to_fixed(v2.y);
-  const long long w0 = to_fixed(v0.w), w1 = to_fixed(v1.w), w2 = to_fixed(v2.w);
-  m[0] = wsub(wmul(y1, w2), wmul(w1, y2));
-  m[1] = wsub(wmul(x2, w1), wmul(w2, x1));
-  m[2] = wsub(wmul(x1, y2), wmul(y1, x2));
-  m[3] = wsub(wmul(y2, w0), wmul(w2, y0));
-  m[4] = wsub(wmul(x0, w2), wmul(w0, x2));
-  m[5] = wsub(wmul(x2, y0), wmul(y2, x0));
-  m[6] = wsub(wmul(y0, w1), wmul(w0, y1));
-  m[7] = wsub(wmul(x1, w0), wmul(w1, x0));
-  m[8] = wsub(wmul(x0, y1), wmul(y0, x1));
+// `small`: fits_fixed32 of the vertices.
+__device__ __forceinline__ void edge_matrix(float4 v0, float4 v1, float4 v2, int culling,
+                                            bool small, long long m[9]) {
+  long long x0, x1, x2;
+  if (small) {  // 32 x 32 -> 64 bit multiply-adds
+    const auto fix = [](float f) { return __float2int_rz(__fmul_rn(f, 65536.0f)); };
+    const int a0 = fix(v0.x), a1 = fix(v1.x), a2 = fix(v2.x);
+    const int y0 = fix(v0.y), y1 = fix(v1.y), y2 = fix(v2.y);
+    const int w0 = fix(v0.w), w1 = fix(v1.w), w2 = fix(v2.w);
+    const auto det2 = [](int a, int b, int c, int d) {
+      return (long long)a * b - (long long)c * d;
+    };
+    m[0] = det2(y1, w2, w1, y2);
+    m[1] = det2(a2, w1, w2, a1);
+    m[2] = det2(a1, y2, y1, a2);
+    m[3] = det2(y2, w0, w2, y0);
+    m[4] = det2(a0, w2, w0, a2);
+    m[5] = det2(a2, y0, y2, a0);
+    m[6] = det2(y0, w1, w0, y1);
+    m[7] = det2(a1, w0, w1, a0);
+    m[8] = det2(a0, y1, y0, a1);
+    x0 = a0; x1 = a1; x2 = a2;
+  } else {
+    const long long y0 = to_fixed(v0.y), y1 = to_fixed(v1.y), y2 = to_fixed(v2.y);
+    const long long w0 = to_fixed(v0.w), w1 = to_fixed(v1.w), w2 = to_fixed(v2.w);
+    x0 = to_fixed(v0.x); x1 = to_fixed(v1.x); x2 = to_fixed(v2.x);
+    m[0] = wsub(wmul(y1, w2), wmul(w1, y2));
+    m[1] = wsub(wmul(x2, w1), wmul(w2, x1));
+    m[2] = wsub(wmul(x1, y2), wmul(y1, x2));
+    m[3] = wsub(wmul(y2, w0), wmul(w2, y0));
+    m[4] = wsub(wmul(x0, w2), wmul(w0, x2));
+    m[5] = wsub(wmul(x2, y0), wmul(y2, x0));
+    m[6] = wsub(wmul(y0, w1), wmul(w0, y1));
+    m[7] = wsub(wmul(x1, w0), wmul(w1, x0));
+    m[8] = wsub(wmul(x0, y1), wmul(y0, x1));
+  }
   if (culling == DR_CULL_NONE || culling == DR_CULL_FRONT) {
     const long long det_i = wadd(wadd(wmul(x0, m[0]), wmul(x1, m[3])), wmul(x2, m[6]));
-    const float det = __ll2float_rn(det_i);
+    const float det = ll_to_float_rn(det_i);
     const float sign = culling == DR_CULL_NONE ? copysignf(1.0f, det) : -1.0f;
 #pragma unroll
-    for (int i = 0; i < 9; ++i) m[i] = __float2ll_rz(__fmul_rn(__ll2float_rn(m[i]), sign));
+    for (int i = 0; i < 9; ++i) m[i] = float_to_ll_rz(__fmul_rn(ll_to_float_rn(m[i]), sign));
   }
 }
 

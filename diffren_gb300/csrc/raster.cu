@@ -9,7 +9,6 @@
 // pixel keeps the L smallest packed (depth | triangle id) keys, which is
 // independent of the order fragments arrive in.
 #include <algorithm>
-#include <cstddef>
 #include <cstring>
 #include <string>
 
@@ -29,24 +28,28 @@ constexpr int kThreads = 128;
 constexpr int kDefaultTile = 16;
 constexpr int kDefaultLargeTiles = 16;
 
+// What setup keeps of a triangle: its clip vertices and vertex indices, 64
+// bytes in four 16-byte loads. With back-face culling the edge coefficients
+// (72 bytes) are recomputed from it where they are needed, in about 50
+// instructions: a scattered load costs an L1 cycle per lane, and nine of them
+// per sample bounded the epilogue, as their stores did setup. The other
+// culling modes round each coefficient to float precision, which costs three
+// times that: setup keeps theirs (RasterArgs::edges). With 144-byte records
+// of everything the fine kernel took 313 us on a 200k-triangle soup
+// (8 x 512^2), 629 on the 4 x 2048^2 terrain and 1025 on the 64-mesh ragged
+// batch, now 244, 548 and 974; setup 109, 227 and 137 us, now 94, 141 and 116.
 struct __align__(16) TriSetup {
-  long long m[9];  // edge-function coefficients (unnormalized inverse)
-  float vz[3];     // clip z of the three vertices
-  float vw[3];     // clip w of the three vertices
-  // The rest serves the fused epilogue only (the fine loop stages the first
-  // 96 bytes): vertex indices and clip x, y, so that a sample's
-  // interpolation reads one record instead of gathering its triangle and
-  // vertices.
+  float4 v[3];
   int32_t vid[3];
-  float vx[3];
-  float vy[3];
-  int32_t pad[3];
+  int32_t small;  // the coordinates fit 32 bits in fixed point (fits_fixed32)
 };
-static_assert(sizeof(TriSetup) == 144, "TriSetup layout");
-static_assert(offsetof(TriSetup, vz) == 72 && offsetof(TriSetup, vw) == 84 &&
-                  offsetof(TriSetup, vid) == 96 && offsetof(TriSetup, vx) == 108 &&
-                  offsetof(TriSetup, vy) == 120,
-              "write_sample reads the record by these offsets");
+static_assert(sizeof(TriSetup) == 64, "TriSetup layout");
+
+// Workspace taken per triangle for the record and the coefficients; rounded
+// up so that what a caller's or the static scratch's fixed size admits does
+// not move with their layout.
+constexpr size_t kSetupBytes = 144;
+static_assert(sizeof(TriSetup) + 5 * sizeof(longlong2) <= kSetupBytes, "setup workspace");
 
 struct RasterArgs {
   const float4* verts;
@@ -59,6 +62,7 @@ struct RasterArgs {
   int32_t total_tiles;
   int scan_shift;  // tiles per block of tile_scan_kernel, as a power of two
   TriSetup* setup;
+  longlong2* edges;  // [tris][5] (the tenth unused), for DR_CULL_NONE / FRONT
   uint2* box;   // left | right << 16, bottom | top << 16; empty when culled
   int2* place;  // inside one tile: {tile, slot}; in 2..large_tiles tiles:
                 // {-2, -}; otherwise {-1, -}
@@ -99,7 +103,7 @@ Layout make_layout(int64_t tris, int64_t tiles, int images, int large_tiles) {
   l.large_count = o; o = align_up(o + 4 * size_t(images));
   l.zero_end = o;
   l.tile_first = o; o = align_up(o + 4 * (tiles + 1));
-  l.setup = o; o = align_up(o + sizeof(TriSetup) * tris);
+  l.setup = o; o = align_up(o + kSetupBytes * tris);
   l.box = o; l.place = o + 8 * tris; o = align_up(o + 16 * tris);
   l.bins = o; o = align_up(o + 4 * size_t(large_tiles) * tris);
   l.large_list = o; o = align_up(o + 4 * tris);
@@ -155,6 +159,21 @@ __device__ __forceinline__ int tile_end(const RasterArgs& a, int i) {
                                                       : a.tile_first[i + 1];
 }
 
+// Edge coefficients of a triangle that setup kept.
+__device__ __forceinline__ void load_edges(const RasterArgs& a, int64_t g, const float4 (&v)[3],
+                                           bool small, long long m[9]) {
+  if (a.culling == DR_CULL_BACK) {
+    edge_matrix(v[0], v[1], v[2], DR_CULL_BACK, small, m);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const longlong2 e = __ldg(a.edges + 5 * g + k);
+      m[2 * k] = e.x;
+      if (k < 4) m[2 * k + 1] = e.y;
+    }
+  }
+}
+
 // One thread per triangle of the batch: bounding box, edge matrix, exact
 // coverage cull, per-tile counts (small triangles) or the large list.
 // Bounded to 64 registers so that 32 warps share an SM: the kernel waits on
@@ -188,20 +207,21 @@ __global__ void __launch_bounds__(128, 8) setup_kernel(RasterArgs a, Batch B) {
     const bool disc = a.depth_mode == DR_DEPTH_DISCRETIZED;
     valid = triangle_box(v0, v1, v2, W, H, box, disc);
     if (valid) {
-      TriSetup s;
-      edge_matrix(v0, v1, v2, a.culling, s.m);
-      valid = !cannot_cover(s.m, box, W, H, disc);
+      long long m[9];
+      const bool small = fits_fixed32(v0, v1, v2);
+      edge_matrix(v0, v1, v2, a.culling, small, m);
+      valid = !cannot_cover(m, box, W, H, disc);
       if (valid) {
-        s.vz[0] = v0.z; s.vz[1] = v1.z; s.vz[2] = v2.z;
-        s.vw[0] = v0.w; s.vw[1] = v1.w; s.vw[2] = v2.w;
-        s.vid[0] = i0; s.vid[1] = i1; s.vid[2] = i2;
-        s.vx[0] = v0.x; s.vx[1] = v1.x; s.vx[2] = v2.x;
-        s.vy[0] = v0.y; s.vy[1] = v1.y; s.vy[2] = v2.y;
-        s.pad[0] = s.pad[1] = s.pad[2] = 0;
-        const int4* src = reinterpret_cast<const int4*>(&s);
-        int4* dst = reinterpret_cast<int4*>(a.setup + g);
+        TriSetup* t = a.setup + g;
+        t->v[0] = v0;
+        t->v[1] = v1;
+        t->v[2] = v2;
+        *reinterpret_cast<int4*>(t->vid) = make_int4(i0, i1, i2, small);
+        if (a.culling != DR_CULL_BACK) {
 #pragma unroll
-        for (int k = 0; k < 9; ++k) dst[k] = src[k];
+          for (int k = 0; k < 5; ++k)
+            a.edges[5 * g + k] = make_longlong2(m[2 * k], k < 4 ? m[2 * k + 1] : 0);
+        }
       }
     }
   }
@@ -470,26 +490,14 @@ __device__ __forceinline__ void row_coefficients(const long long* m, float* row,
 // A depth of exactly 1 is background: its attributes stay as
 // fill_background left them.
 __device__ __forceinline__ void write_sample(const RasterArgs& a, const Batch& B, int img,
-                                          const TriSetup* t, int4 r4, float zz,
+                                          int4 vid, const float4 (&v)[3], float zz,
                                           const float b[3], int64_t o) {
   const SampleOutputs& so = a.so;
   const int K = so.K;
   const bool vec_rows = (K & 3) == 0;
   if (zz == 1.0f) return;
-  // One record holds the vertex indices and clip coordinates; r4 is its
-  // fifth 16 bytes.
-  const float2 z01 = make_float2(__int_as_float(r4.z), __int_as_float(r4.w));
-  const int4 r5 = __ldg(reinterpret_cast<const int4*>(t) + 5);  // vz2, vw0..2
-  const int4 r6 = __ldg(reinterpret_cast<const int4*>(t) + 6);  // vid0..2, vx0
-  const int4 r7 = __ldg(reinterpret_cast<const int4*>(t) + 7);  // vx1, vx2, vy0, vy1
-  const int4 r8 = __ldg(reinterpret_cast<const int4*>(t) + 8);  // vy2
-  const int v0 = r6.x, v1 = r6.y, v2 = r6.z;
-  const float4 c = lerp_clip(make_float4(__int_as_float(r6.w), __int_as_float(r7.z), z01.x,
-                                         __int_as_float(r5.y)),
-                             make_float4(__int_as_float(r7.x), __int_as_float(r7.w), z01.y,
-                                         __int_as_float(r5.z)),
-                             make_float4(__int_as_float(r7.y), __int_as_float(r8.x),
-                                         __int_as_float(r5.x), __int_as_float(r5.w)), b);
+  const int v0 = vid.x, v1 = vid.y, v2 = vid.z;
+  const float4 c = lerp_clip(v[0], v[1], v[2], b);
   if (so.attr) {
     float* ao = so.attr_out + o * K;
     const float* ab = so.attr + B.vertex_offset[img] * K;
@@ -746,18 +754,16 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
       const int total = tot & 0xfffff, ntri = tot >> 20;
       if (cnt > 0) {
         const int slot = excl >> 20, off = excl & 0xfffff;
-        int4 r[6];
-        const int4* src = reinterpret_cast<const int4*>(a.setup + g);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) r[k] = __ldg(src + k);
-        const long long* mm = reinterpret_cast<const long long*>(r);
-        const float* ff = reinterpret_cast<const float*>(r) + 18;
+        const TriSetup* st = a.setup + g;
+        const float4 v[3] = {__ldg(st->v), __ldg(st->v + 1), __ldg(st->v + 2)};
+        long long mm[9];
+        load_edges(a, g, v, __ldg(&st->small), mm);
 #pragma unroll
         for (int k = 0; k < 9; ++k) s.m[k * kThreads + slot] = mm[k];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          s.vz[k * kThreads + slot] = ff[k];
-          s.vw[k * kThreads + slot] = ff[3 + k];
+          s.vz[k * kThreads + slot] = v[k].z;
+          s.vw[k * kThreads + slot] = v[k].w;
         }
         s.tid[slot] = int(g - tri0);
         row_coefficients(mm, s.row, slot);
@@ -908,14 +914,10 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
       float b[3] = {0.0f, 0.0f, 0.0f};
       const int id = int(uint32_t(key));
       const TriSetup* st = a.setup + tri0 + id;
-      // The coefficients in 16-byte loads (the record's first 72 bytes; the
-      // fifth load also brings two of the depths).
-      int4 r[5];
-#pragma unroll
-      for (int k = 0; k < 5; ++k) r[k] = __ldg(reinterpret_cast<const int4*>(st) + k);
+      const float4 v[3] = {__ldg(st->v), __ldg(st->v + 1), __ldg(st->v + 2)};
+      const int4 vid = __ldg(reinterpret_cast<const int4*>(st->vid));
       long long m[9];
-#pragma unroll
-      for (int k = 0; k < 9; ++k) m[k] = reinterpret_cast<const long long*>(r)[k];
+      load_edges(a, tri0 + id, v, vid.w, m);
       long long e[3];
       edge_values(m, s.pxf[lx], s.pyf[ly], e);
       float bb[3];
@@ -924,8 +926,8 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
       if (disc) {
         zz = undiscretize_z(uint32_t(key >> 32));
       } else {
-        const float3 vz = make_float3(__ldg(&st->vz[0]), __ldg(&st->vz[1]), __ldg(&st->vz[2]));
-        const float3 vw = make_float3(__ldg(&st->vw[0]), __ldg(&st->vw[1]), __ldg(&st->vw[2]));
+        const float3 vz = make_float3(v[0].z, v[1].z, v[2].z);
+        const float3 vw = make_float3(v[0].w, v[1].w, v[2].w);
         zz = fragment_z(bb, vz, vw, false);
       }
       if (!disc || zz != 1.0f) { b[0] = bb[0]; b[1] = bb[1]; b[2] = bb[2]; }
@@ -935,7 +937,7 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
       bo[0] = b[0];
       bo[1] = b[1];
       bo[2] = b[2];
-      if (kFused) write_sample(a, B, img, st, r[4], zz, b, o);
+      if (kFused) write_sample(a, B, img, vid, v, zz, b, o);
     }
     __syncthreads();
   }
@@ -1113,6 +1115,7 @@ int raster_launch(const float* vertices, const int32_t* triangles,
     a.scan_shift = 12;  // 4096 tiles per block, more above 32 blocks
     while (((int64_t(tiles) + (int64_t(1) << a.scan_shift) - 1) >> a.scan_shift) > 32) ++a.scan_shift;
     a.setup = reinterpret_cast<TriSetup*>(ws + lay.setup);
+    a.edges = reinterpret_cast<longlong2*>(ws + lay.setup + sizeof(TriSetup) * size_t(tris));
     a.box = reinterpret_cast<uint2*>(ws + lay.box);
     a.place = reinterpret_cast<int2*>(ws + lay.place);
     a.tile_count = reinterpret_cast<int32_t*>(ws + lay.tile_count);
