@@ -1,0 +1,44 @@
+"""The texture kernels at the edges of their dispatch: one to five channels,
+point counts around a block's, buffers off the wide loads' alignment."""
+import numpy as np
+import pytest
+import torch
+
+from diffren_gb300 import shaders
+from oracle import texture
+
+pytestmark = pytest.mark.gpu
+
+
+def _at_offset(a, floats, device):
+  """A contiguous CUDA copy of `a` that starts `floats` floats into its storage."""
+  buf = torch.empty(a.size + floats, dtype=torch.float32, device=device)
+  out = buf[floats:].view(a.shape)
+  out.copy_(torch.tensor(a))
+  return out
+
+
+@pytest.mark.parametrize("channels", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("points", [1, 255, 257, 511, 512, 513, 1025])
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_texture_dispatch(channels, points, offset, device):
+  rng = np.random.default_rng(points + channels)
+  tex = rng.uniform(-1, 1, (6, 9, channels)).astype(np.float32)
+  uv = rng.uniform(-0.2, 1.2, (points, 2)).astype(np.float32)
+  g = rng.standard_normal((points, channels)).astype(np.float32)
+  g[::5] = 0.0  # points without gradient
+  g[1::7, 0] = 0.0  # and channels
+  du = _at_offset(uv, offset, device).requires_grad_()
+  dt = _at_offset(tex, offset, device).requires_grad_()
+  out = shaders.texture_map(du, dt)
+  np.testing.assert_array_equal(out.detach().cpu().numpy(), texture.texture_map(uv, tex))
+  got = torch.autograd.grad(out, (du, dt), _at_offset(g, offset, device))
+  tu = torch.tensor(uv, dtype=torch.float64, requires_grad=True)
+  tt = torch.tensor(tex, dtype=torch.float64, requires_grad=True)
+  want = torch.autograd.grad(texture.texture_map_t(tu, tt), (tu, tt),
+                             torch.tensor(g, dtype=torch.float64))
+  # A texel sums up to 4 points / 54 texels of products of three rounded
+  # factors, a coordinate channels x 2 of them times 9: below 1e-4 of the
+  # largest magnitude.
+  for x, y in zip(got, want):
+    assert (x.cpu().double() - y).abs().max() <= 1e-4 * y.abs().max()
