@@ -540,9 +540,10 @@ struct SplatArgs {
   int64_t P;     // pixels covered by the call: plane stride of `saved`
   float coef;
   float* out;
-  float* saved;  // [3 (C+1) + 2, P] planar accumulators, surface codes and
-                 // the tile list (forward out; the backward reads it and
-                 // resets its own work counter in it)
+  float* saved;  // [3 (C+1) + 2, P] accumulators, surface codes and the tile
+                 // list (forward out; the backward reads it and resets its
+                 // own work counter in it): planes of one value, or of four
+                 // (see saved_wide)
   float* accum;
   float* normalized;
   const float* d_out;
@@ -550,6 +551,14 @@ struct SplatArgs {
   float4* d_vp;
   bool fg_grads;  // DR_SPLAT_FOREGROUND_GRADIENTS: background d_colors unwritten
 };
+
+// Four channels and a 16-byte aligned buffer: the 15 accumulators and the
+// code of a pixel are four float4 planes, so that a pixel takes 4 stores and 4
+// loads instead of 16 of each.
+template <int C>
+__device__ __forceinline__ bool saved_wide(const SplatArgs& a) {
+  return C == 4 && (reinterpret_cast<uintptr_t>(a.saved) & 15) == 0;
+}
 
 // A block covers a kTX x kTY tile of pixels, one per thread; the samples it
 // reads are the tile plus a 1-pixel halo: kRS x (kTY + 2) per layer.
@@ -983,13 +992,23 @@ __device__ __forceinline__ void splat_fwd_tile(const SplatArgs& a, const Batch& 
   // foreground samples next to it, and every such sample lies in this
   // tile's region: a region without foreground leaves them unwritten.
   if (a.saved && layers != 0) {
+    if (saved_wide<C>(a)) {
+      if constexpr (C == 4) {
+        float4* q = reinterpret_cast<float4*>(a.saved) + pix;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
+        for (int k = 0; k < 3; ++k)
+          q[k * a.P] = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+        q[3 * a.P] = make_float4(wacc[0], wacc[1], wacc[2], __uint_as_float(code));
+      }
+    } else {
 #pragma unroll
-      for (int c = 0; c < C; ++c) a.saved[(k * (C + 1) + c) * a.P + pix] = acc[k][c];
-      a.saved[(k * (C + 1) + C) * a.P + pix] = wacc[k];
+      for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) a.saved[(k * (C + 1) + c) * a.P + pix] = acc[k][c];
+        a.saved[(k * (C + 1) + C) * a.P + pix] = wacc[k];
+      }
+      if (LT == 3) reinterpret_cast<unsigned*>(a.saved)[3 * (C + 1) * a.P + pix] = code;
     }
-    if (LT == 3) reinterpret_cast<unsigned*>(a.saved)[3 * (C + 1) * a.P + pix] = code;
   }
   if (a.accum || a.normalized) {
     const int64_t HW = int64_t(W) * H;
@@ -1195,11 +1214,28 @@ __device__ __forceinline__ void splat_bwd_tile(const SplatArgs& a, const Batch& 
     if (qx >= 0 && qy >= 0 && qx < W && qy < H) {
       const int64_t pix = B.pix_off[tr.img] + int64_t(qy) * W + qx;
       float acc[3][C], wacc[3];
+      unsigned code = 0;
+      if (saved_wide<C>(a)) {
+        if constexpr (C == 4) {
+          const float4* q = reinterpret_cast<const float4*>(a.saved) + pix;
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
+          for (int k = 0; k < 3; ++k) {
+            const float4 v = __ldg(q + k * a.P);
+            acc[k][0] = v.x; acc[k][1] = v.y; acc[k][2] = v.z; acc[k][3] = v.w;
+          }
+          const float4 v = __ldg(q + 3 * a.P);
+          wacc[0] = v.x; wacc[1] = v.y; wacc[2] = v.z;
+          code = __float_as_uint(v.w);
+        }
+      } else {
 #pragma unroll
-        for (int c = 0; c < C; ++c) acc[k][c] = __ldg(a.saved + (k * (C + 1) + c) * a.P + pix);
-        wacc[k] = __ldg(a.saved + (k * (C + 1) + C) * a.P + pix);
+        for (int k = 0; k < 3; ++k) {
+#pragma unroll
+          for (int c = 0; c < C; ++c) acc[k][c] = __ldg(a.saved + (k * (C + 1) + c) * a.P + pix);
+          wacc[k] = __ldg(a.saved + (k * (C + 1) + C) * a.P + pix);
+        }
+        if (LT == 3 && a.zb)
+          code = __ldg(reinterpret_cast<const unsigned*>(a.saved) + 3 * (C + 1) * a.P + pix);
       }
       float d[C];
       load_row<C>(a.d_out + pix * C, d);
@@ -1208,8 +1244,7 @@ __device__ __forceinline__ void splat_bwd_tile(const SplatArgs& a, const Batch& 
       if (LT == 3 && a.zb) {
         // The forward's surface codes of this pixel's taps replace the
         // depths (the zs area holds them).
-        reinterpret_cast<unsigned*>(zs)[i] =
-            __ldg(reinterpret_cast<const unsigned*>(a.saved) + 3 * (C + 1) * a.P + pix);
+        reinterpret_cast<unsigned*>(zs)[i] = code;
       } else if (a.zb) {
         unsigned m = 0;
         for (int l = 0; l < L; ++l) m |= unsigned(__ldg(a.zb + eq + l * HW) != 1.0f) << l;

@@ -486,11 +486,13 @@ int dr_vertex_normals_csr_bwd(const float* d_normals, const float* vertices,
  * foreground flag. colors [L, H, W, C]
  * (1 <= C <= DR_MAX_SPLAT_CHANNELS, last channel alpha); out [H, W, C].
  * saved [3 (C + 1) + 2, P] receives the fg/surface/bg accumulators and
- * weights the VJP needs, one plane of P pixels per value, P = the largest
- * pixel_offset + width * height of the images, then (for three layers) each
- * pixel's surface classes of its 9 taps as 32-bit codes, then the list of
- * the screen tiles that hold foreground (nullable; the planes are written
- * only near foreground samples, where dr_splat_bwd reads them); accum and
+ * weights the VJP needs and (for three layers) each pixel's surface classes
+ * of its 9 taps as a 32-bit code, P = the largest pixel_offset + width *
+ * height of the images, then the list of the screen tiles that hold
+ * foreground: one plane of P pixels per value, or, for four channels in a
+ * 16-byte aligned buffer, four planes of 16 bytes per pixel (nullable; the
+ * planes are written only near foreground samples, where dr_splat_bwd reads
+ * them; the buffer belongs to the library between the calls); accum and
  * normalized [3, H, W, C] are
  * the reference's debugging buffers (nullable). With C % 4 == 0 the color
  * and output buffers must be 16-byte aligned. */

@@ -93,3 +93,37 @@ def test_samples_vjp_block_rule(sizes, layers, channels, deterministic, device):
   want = _reference(attr.detach(), clip.detach(), bary[fg], vid, wh, g_attr[fg], g_pos[fg])
   for x, y in zip(got, want):
     assert (x.double() - y).abs().max() <= 1e-4 * y.abs().max()
+
+
+# Four channels in a 16-byte aligned buffer save float4 planes, anything else
+# one plane per value; both hold the same numbers.
+@pytest.mark.parametrize("layers", [1, 2, 3])
+@pytest.mark.parametrize("listed", [True, False])
+def test_saved_planes_aligned_and_not(layers, listed, device):
+  w, h, C = 83, 37, 4
+  g = torch.Generator(device=device).manual_seed(layers)
+  rand = lambda *s: torch.rand(*s, generator=g, device=device)
+  fg = torch.arange(layers, device=device)[:, None, None] < (rand(h, w) * (layers + 1)).long()
+  z = torch.where(fg, 0.5, 1.0).contiguous()
+  pos = torch.zeros(layers, h, w, 4, device=device)
+  pos[..., 0] = torch.arange(w, device=device) + rand(layers, h, w)
+  pos[..., 1] = torch.arange(h, device=device)[:, None] + rand(layers, h, w)
+  pos[..., 2] = torch.where(fg, rand(layers, h, w), 1.0)
+  pos[..., 3] = fg.float()
+  colors = rand(layers, h, w, C)
+  d_out = torch.randn(h, w, C, generator=g, device=device)
+  batch = kernels.ImageBatch.single(w, h, 0, 0)
+  lib, P, st = _lib.load(), kernels._p, kernels._stream(device)
+  zb = z if listed else None
+  results = []
+  for offset in (0, 1):
+    saved = torch.empty((3 * (C + 1) + 2) * w * h + 1, device=device)[offset:]
+    out = torch.empty(h, w, C, device=device)
+    d_c, d_p = torch.zeros_like(colors), torch.zeros_like(pos)
+    assert lib.dr_splat_fwd(P(pos), P(zb), P(colors), C, batch.ptr, 1, layers, P(out), P(saved),
+                            None, None, st) == 0
+    assert lib.dr_splat_bwd(P(d_out), P(pos), P(zb), P(colors), P(saved), C, batch.ptr, 1, layers,
+                            P(d_c), P(d_p), st) == 0
+    results.append((out, d_c, d_p))
+  for a, b in zip(*results):
+    assert torch.equal(a, b) and torch.count_nonzero(a) > 0
