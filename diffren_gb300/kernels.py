@@ -9,8 +9,8 @@ current CUDA stream go to the library through ctypes. The ops work on packed
 ragged batches described by an ``ImageBatch``; a single image is a batch of
 one.
 """
-import contextlib
 import ctypes
+import itertools
 import threading
 
 import numpy as np
@@ -34,18 +34,47 @@ LAUNCHES = _LaunchCounter()
 _PROFILE = None  # list of (op, start event, end event) while profiling
 
 
-@contextlib.contextmanager
+class _NoContext:
+  """A with-statement that does nothing (contextlib's costs 2 us a call)."""
+  __slots__ = ()
+
+  def __enter__(self):
+    pass
+
+  def __exit__(self, *exc):
+    pass
+
+
+class _Timed:
+  """CUDA events around one op while profiling."""
+
+  def __init__(self, name):
+    self.name = name
+
+  def __enter__(self):
+    self.e0 = torch.cuda.Event(enable_timing=True)
+    self.e1 = torch.cuda.Event(enable_timing=True)
+    self.e0.record()
+
+  def __exit__(self, exc_type, *_):
+    if exc_type is None:
+      self.e1.record()
+      _PROFILE.append((self.name, self.e0, self.e1))
+
+
+_NO_CONTEXT = _NoContext()
+
+
 def _op(name, kernels_launched):
   LAUNCHES.count += kernels_launched
-  if _PROFILE is None:
-    yield
-    return
-  e0 = torch.cuda.Event(enable_timing=True)
-  e1 = torch.cuda.Event(enable_timing=True)
-  e0.record()
-  yield
-  e1.record()
-  _PROFILE.append((name, e0, e1))
+  return _NO_CONTEXT if _PROFILE is None else _Timed(name)
+
+
+def _on_device(device):
+  """Makes `device` current for a block, where it is not already."""
+  if device.index == torch.cuda.current_device():
+    return _NO_CONTEXT
+  return torch.cuda.device(device)
 
 
 def profile_step(step, steps, device):
@@ -70,19 +99,28 @@ def _groups(batch):
 
 
 def _p(t):
-  return None if t is None else ctypes.c_void_p(t.data_ptr())
+  """A tensor's address (the entry points' argument types make it void*)."""
+  return None if t is None else t.data_ptr()
 
 
 def _stream(device=None):
-  return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+  """Handle of the current stream of a device (torch.device or None)."""
+  index = None if device is None else device.index
+  if index is None:
+    index = torch.cuda.current_device()
+  return torch._C._cuda_getCurrentRawStream(index)
 
 
 def _f32(t, device=None):
+  if device is None and isinstance(t, torch.Tensor) and t.dtype == torch.float32:
+    return t.contiguous()
   t = torch.as_tensor(t, dtype=torch.float32, device=device)
   return t.contiguous()
 
 
 def _i32(t, device=None):
+  if device is None and isinstance(t, torch.Tensor) and t.dtype == torch.int32:
+    return t.contiguous()
   t = torch.as_tensor(t, device=device)
   return t.to(torch.int32).contiguous()
 
@@ -116,21 +154,19 @@ class ImageBatch:
     for w, h in zip(self.widths, self.heights):
       if w <= 0 or h <= 0:
         raise ValueError("image width and height must be > 0")
-    self.pixel_offsets = np.concatenate(
-        [[0], np.cumsum([w * h for w, h in zip(self.widths, self.heights)])])
-    self.vertex_offsets = np.concatenate([[0], np.cumsum(self.num_vertices)])
-    self.triangle_offsets = np.concatenate([[0], np.cumsum(self.num_triangles)])
+    pixels = [w * h for w, h in zip(self.widths, self.heights)]
+    offsets = [list(itertools.accumulate(x, initial=0))
+               for x in (pixels, self.num_vertices, self.num_triangles)]
+    self.pixel_offsets, self.vertex_offsets, self.triangle_offsets = (
+        np.array(x, dtype=np.int64) for x in offsets)
     self.total_pixels = int(self.pixel_offsets[-1])
     self.total_vertices = int(self.vertex_offsets[-1])
     self.total_triangles = int(self.triangle_offsets[-1])
-    self.descs = (ImageDesc * max(n, 1))()
-    for i in range(n):
-      d = self.descs[i]
-      d.width, d.height = self.widths[i], self.heights[i]
-      d.num_vertices, d.num_triangles = self.num_vertices[i], self.num_triangles[i]
-      d.vertex_offset = int(self.vertex_offsets[i])
-      d.triangle_offset = int(self.triangle_offsets[i])
-      d.pixel_offset = int(self.pixel_offsets[i])
+    self.descs = (ImageDesc * max(n, 1))(*(
+        ImageDesc(width=w, height=h, num_vertices=v, num_triangles=t, vertex_offset=vo,
+                  triangle_offset=to, pixel_offset=po)
+        for w, h, v, t, po, vo, to in zip(self.widths, self.heights, self.num_vertices,
+                                          self.num_triangles, *offsets)))
 
   def vertex_image_index(self, device):
     """[sum V] int64 image index of every packed vertex (cached per device)."""
@@ -147,7 +183,7 @@ class ImageBatch:
 
   @property
   def ptr(self):
-    return ctypes.cast(self.descs, ctypes.c_void_p)
+    return ctypes.addressof(self.descs)
 
   def layered_view(self, flat, i, num_layers):
     """[L, H_i, W_i, ...] view of image i of a packed layered buffer."""
@@ -203,7 +239,7 @@ _workspaces = {}
 
 
 def default_workspace(device):
-  key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+  key = (device.index, _stream(device))
   with _ws_lock:
     ws = _workspaces.get(key)
     if ws is None:
@@ -239,7 +275,7 @@ def rasterize_packed(clip, triangles, batch, config, workspace=None, out=None):
     ids, z, bary = out
   need = raster_workspace_bytes(batch, config)
   ws = (workspace or default_workspace(dev)).get(need)
-  with torch.cuda.device(dev), _op("raster", 5 * _groups(batch)):
+  with _on_device(dev), _op("raster", 5 * _groups(batch)):
     rc = lib.dr_rasterize_batch(_p(clip), _p(triangles), batch.ptr, batch.n,
                                 ctypes.byref(config), _p(ids), _p(z), _p(bary),
                                 _p(ws), ws.numel(), _stream(dev))
@@ -614,7 +650,7 @@ class _RasterSamples(torch.autograd.Function):
     vp = torch.empty(n, 4, dtype=torch.float32, device=dev)
     vids = None if recompute else torch.empty(n, 3, dtype=torch.int32, device=dev)
     ws = workspace.get(raster_workspace_bytes(batch, config))
-    with torch.cuda.device(dev), _op("raster", 5 * _groups(batch)):
+    with _on_device(dev), _op("raster", 5 * _groups(batch)):
       rc = lib.dr_rasterize_batch_interpolate(
           _p(clip), _p(triangles), batch.ptr, batch.n, ctypes.byref(config), _p(ids), _p(z),
           _p(bary), _p(attributes), K, _p(out), _p(vp), _p(vids), _p(ws), ws.numel(),
@@ -678,7 +714,7 @@ def _rerasterize(ctx, clip, triangles):
   vp = torch.empty(n, 4, dtype=torch.float32, device=dev)
   vids = torch.empty(n, 3, dtype=torch.int32, device=dev)
   ws = ctx.workspace.get(raster_workspace_bytes(ctx.batch, ctx.config))
-  with torch.cuda.device(dev), _op("raster_recompute", 5 * _groups(ctx.batch)):
+  with _on_device(dev), _op("raster_recompute", 5 * _groups(ctx.batch)):
     rc = lib.dr_rasterize_batch_interpolate(
         _p(clip), _p(triangles), ctx.batch.ptr, ctx.batch.n, ctypes.byref(ctx.config),
         _p(ids), _p(z), _p(bary), None, 0, None, _p(vp), _p(vids), _p(ws), ws.numel(),

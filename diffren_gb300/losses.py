@@ -31,7 +31,7 @@ def squared_error_seed(image, target, weight=1.0):
                          device=image.device)
   loss = torch.empty((), dtype=torch.float32, device=image.device)
   lib = _lib.load()
-  with torch.cuda.device(image.device), kernels._op("squared_error", 2):
+  with kernels._on_device(image.device), kernels._op("squared_error", 2):
     rc = lib.dr_squared_error(kernels._p(image), kernels._p(target), image.numel(),
                               float(weight), kernels._p(seed), kernels._p(partials),
                               kernels._p(loss), kernels._stream(image.device))

@@ -77,16 +77,21 @@ class Geometry:
     T = triangles.shape[-2]
     self.batch = kernels.ImageBatch([image_width] * B, [image_height] * B, [V] * B,
                                     [T] * B)
-    v = vertices.expand(B, *vertices.shape[-2:]) if vertices.dim() == 2 else vertices
-    self.world = v.reshape(B * V, vertices.shape[-1]).float()
-    t = triangles.expand(B, T, 3) if triangles.dim() == 2 else triangles
-    self.triangles_packed = t.reshape(B * T, 3).to(torch.int32).contiguous()
+    if self.batched:
+      v = vertices.expand(B, *vertices.shape[-2:]) if vertices.dim() == 2 else vertices
+      t = triangles.expand(B, T, 3) if triangles.dim() == 2 else triangles
+      v, t = v.reshape(B * V, vertices.shape[-1]), t.reshape(B * T, 3)
+      if camera is not None and camera.dim() == 2:
+        camera = camera.expand(B, 4, 4)
+    else:
+      v, t = vertices, triangles
+    self.world = v.float()
+    self.triangles_packed = t.to(torch.int32).contiguous()
     self.triangles = triangles
     if camera is None:
       self.clip = self.world.contiguous()
     else:
-      cam = camera.expand(B, 4, 4) if camera.dim() == 2 else camera
-      self.clip = kernels.transform(self.world.contiguous(), cam.float(), self.batch)
+      self.clip = kernels.transform(self.world.contiguous(), camera.float(), self.batch)
 
 
 def rasterize_geometry(geom: Geometry, num_layers, face_culling_mode,

@@ -67,16 +67,18 @@ def _render_fused(geom, attributes, shading_function, num_layers, face_culling_m
   interp, vp, ids, z, bary = kernels.rasterize_interpolate_packed(
       cat, geom.clip, geom.triangles_packed, geom.batch, cfg,
       kernels.default_workspace(geom.clip.device), recompute_raster, deterministic_gradients)
-  frame = rasterize.framebuffer_of(geom, num_layers, ids, z, bary)
   lead = (geom.B,) if geom.batched else ()
-  interp = interp.view(*lead, num_layers, frame.height, frame.width, -1)
+  H, W = geom.batch.heights[0], geom.batch.widths[0]
+  interp = interp.view(*lead, num_layers, H, W, -1)
   if passthrough:
     shaded = interp
   else:
     interpolated = dict(zip(keys, kernels.split_channels(interp, widths)))
     shaded = _shade_layers(shading_function, interpolated, num_layers, geom.batched)
-  return splat.splat_positions(vp, frame, shaded, return_accum_buffers,
-                               foreground_gradients=passthrough)
+  colors = splat._shaded_flat(shaded)
+  res = kernels.splat_packed(vp, colors, geom.batch, num_layers, return_accum_buffers, z=z,
+                             foreground_gradients=passthrough)
+  return splat._shape_outputs(res, lead, H, W, colors.shape[1], return_accum_buffers)
 
 
 def render_triangles(vertices, attributes: Dict[str, torch.Tensor], triangles,
