@@ -103,6 +103,7 @@ SIGNATURES = {
                                 _P]),
     "dr_composite_over_fwd": (_I, [_P, _P, _I, _P, _I, _I, _P, _P]),
     "dr_composite_over_bwd": (_I, [_P, _P, _P, _I, _P, _I, _I, _P, _P]),
+    "dr_pack_columns": (_I, [_P, _P, _P, _I, _L, _P, _P]),
     "dr_squared_error": (_I, [_P, _P, _L, _F, _P, _P, _P, _P]),
     "dr_vertex_normals_fwd": (_I, [_P, _P, _P, _I, _P, _P, _P]),
     "dr_vertex_normals_bwd": (_I, [_P, _P, _P, _P, _I, _P, _P, _P, _P]),

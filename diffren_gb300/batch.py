@@ -133,7 +133,7 @@ class BatchRenderer:
       raise ValueError("shading_function=None needs exactly one attribute")
     parts = [kernels._f32(attributes[k], self.device) for k in keys]
     widths = [p.shape[1] for p in parts]
-    cat = torch.cat(parts, dim=1) if len(parts) > 1 else parts[0]
+    cat = kernels.pack_columns(parts)
     splatting = compositing_mode == constants.CompositingMode.SPLAT_OVER
     fused = splatting and cat.shape[1] <= kernels._lib.DR_MAX_CHANNELS
     if self._autotune:

@@ -346,6 +346,14 @@ int dr_composite_over_bwd(const float* d_out, const float* shaded, const float* 
                 err);
 }
 
+int dr_pack_columns(const float* const* parts, const int32_t* widths, const int64_t* strides,
+                    int32_t count, int64_t rows, float* out, void* stream) {
+  std::string err;
+  return finish(dr::pack_columns_launch(parts, widths, strides, count, rows, out,
+                                        as_stream(stream), err),
+                err);
+}
+
 int dr_squared_error(const float* image, const float* target, int64_t count, float weight,
                      float* seed, double* partials, float* loss, void* stream) {
   std::string err;

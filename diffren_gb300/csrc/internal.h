@@ -176,6 +176,10 @@ int over_bwd_launch(const float* d_out, const float* shaded, const float* z, int
                     const dr_image_desc* images, int n, int L, float* d_shaded,
                     cudaStream_t stream, std::string& err);
 
+// columns.cu
+int pack_columns_launch(const float* const* parts, const int32_t* widths, const int64_t* strides,
+                        int count, int64_t n, float* out, cudaStream_t stream, std::string& err);
+
 // loss.cu
 int squared_error_launch(const float* image, const float* target, int64_t n, float weight,
                          float* seed, double* partials, float* loss, cudaStream_t stream,

@@ -34,6 +34,7 @@ struct LightArgs {
   float* d_nrm;
   float* d_pos;
   int sg;  // row stride of the three gradients
+  float* packed;  // the three gradients as columns of one [n, 9] buffer (or null)
 };
 
 struct V3 {
@@ -105,21 +106,16 @@ __global__ void __launch_bounds__(256) point_light_fwd_kernel(LightArgs a) {
   if (a.oc == 4) o[3] = 1.0f;
 }
 
-__global__ void __launch_bounds__(256) point_light_bwd_kernel(LightArgs a) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
+// The gradients of sample i, handed to store(gradient buffer, value).
+template <typename Store>
+__device__ __forceinline__ void light_vjp(const LightArgs& a, int64_t i, const Store& store) {
   const V3 c = load3(a.dif + i * a.sd), n = load3(a.nrm + i * a.sn), p = load3(a.pos + i * a.sp);
   const V3 g = load3(a.d_out + i * a.oc);
   const dr_point_light& q = a.q;
   const Lit s = shade(q, n, p);
   // out_k = c_k luma decay
   const float ld_ = s.luma * s.decay;
-  if (a.d_dif) {
-    float* d = a.d_dif + i * a.sg;
-    d[0] = g.x * ld_;
-    d[1] = g.y * ld_;
-    d[2] = g.z * ld_;
-  }
+  if (a.d_dif) store(a.d_dif, V3{g.x * ld_, g.y * ld_, g.z * ld_});
   if (!a.d_nrm && !a.d_pos) return;
   const float sg = dot(g, c);
   const float d_luma = sg * s.decay, d_decay = sg * s.luma;
@@ -140,19 +136,35 @@ __global__ void __launch_bounds__(256) point_light_bwd_kernel(LightArgs a) {
   V3 d_tl = normalize_vjp(s.tl, s.rl, d_ld);       // ld = normalize(tl)
   if (s.dist > 0.0f) d_tl = add(d_tl, scale(s.tl, d_dist / s.dist));  // dist = |tl|
   const V3 d_te = normalize_vjp(s.te, s.re, d_hs);  // vd = normalize(te)
-  if (a.d_nrm) {
-    float* d = a.d_nrm + i * a.sg;
-    d[0] = d_n.x;
-    d[1] = d_n.y;
-    d[2] = d_n.z;
-  }
-  if (a.d_pos) {  // tl = light - p, te = eye - p
-    float* d = a.d_pos + i * a.sg;
-    d[0] = -d_tl.x - d_te.x;
-    d[1] = -d_tl.y - d_te.y;
-    d[2] = -d_tl.z - d_te.z;
+  if (a.d_nrm) store(a.d_nrm, d_n);
+  if (a.d_pos)  // tl = light - p, te = eye - p
+    store(a.d_pos, V3{-d_tl.x - d_te.x, -d_tl.y - d_te.y, -d_tl.z - d_te.z});
+}
+
+// kPacked: the three gradients fill one [n, 9] buffer (the gradient of a packed
+// attribute buffer); a block's rows go through shared memory and leave as
+// float4s (nine scattered stores per sample took twice the time).
+template <bool kPacked>
+__global__ void __launch_bounds__(256) point_light_bwd_kernel(LightArgs a) {
+  __shared__ __align__(16) float rows[kPacked ? 256 * 9 : 4];
+  const int64_t i0 = int64_t(blockIdx.x) * blockDim.x;
+  const int64_t i = i0 + threadIdx.x;
+  if (i < a.n) light_vjp(a, i, [&](float* base, V3 v) {
+    float* d = kPacked ? rows + 9 * threadIdx.x + (base - a.packed) : base + i * a.sg;
+    d[0] = v.x;
+    d[1] = v.y;
+    d[2] = v.z;
+  });
+  if constexpr (kPacked) {
+    __syncthreads();
+    const int total = int(min(int64_t(256), a.n - i0)) * 9;
+    float* out = a.packed + i0 * 9;
+    for (int k = threadIdx.x; k < total >> 2; k += 256)
+      reinterpret_cast<float4*>(out)[k] = reinterpret_cast<const float4*>(rows)[k];
+    for (int k = (total & ~3) + int(threadIdx.x); k < total; k += 256) out[k] = rows[k];
   }
 }
+
 
 bool check_light(const float* dif, const float* nrm, const float* pos, int64_t n, int sd, int sn,
                  int sp, const dr_point_light* q, int oc, std::string& err) {
@@ -186,7 +198,7 @@ int point_light_fwd_launch(const float* dif, const float* nrm, const float* pos,
     err = "out must be non-null";
     return DR_ERR_INVALID_ARGUMENT;
   }
-  LightArgs a{dif, nrm, pos, n, sd, sn, sp, *q, out, oc, nullptr, nullptr, nullptr, nullptr, 3};
+  LightArgs a{dif, nrm, pos, n, sd, sn, sp, *q, out, oc, nullptr, nullptr, nullptr, nullptr, 3, nullptr};
   point_light_fwd_kernel<<<unsigned((n + 255) / 256), 256, 0, stream>>>(a);
   return launch_status("point light", err);
 }
@@ -205,8 +217,19 @@ int point_light_bwd_launch(const float* d_out, int oc, const float* dif, const f
     err = "gradient row stride must be at least 3 floats";
     return DR_ERR_INVALID_ARGUMENT;
   }
-  LightArgs a{dif, nrm, pos, n, sd, sn, sp, *q, nullptr, oc, d_out, d_dif, d_nrm, d_pos, sg};
-  point_light_bwd_kernel<<<unsigned((n + 255) / 256), 256, 0, stream>>>(a);
+  LightArgs a{dif, nrm, pos, n, sd, sn, sp, *q, nullptr, oc, d_out, d_dif, d_nrm, d_pos, sg, nullptr};
+  if (sg == 9 && d_dif && d_nrm && d_pos) {
+    float* base = std::min(d_dif, std::min(d_nrm, d_pos));
+    const int64_t o[3] = {d_dif - base, d_nrm - base, d_pos - base};
+    if (o[0] != o[1] && o[1] != o[2] && o[0] != o[2] && (reinterpret_cast<uintptr_t>(base) & 15) == 0 &&
+        o[0] <= 6 && o[1] <= 6 && o[2] <= 6 && o[0] % 3 == 0 && o[1] % 3 == 0 && o[2] % 3 == 0)
+      a.packed = base;
+  }
+  const unsigned grid = unsigned((n + 255) / 256);
+  if (a.packed)
+    point_light_bwd_kernel<true><<<grid, 256, 0, stream>>>(a);
+  else
+    point_light_bwd_kernel<false><<<grid, 256, 0, stream>>>(a);
   return launch_status("point light backward", err);
 }
 

@@ -64,7 +64,7 @@ def interpolate_vertex_attributes(attributes: Dict[str, torch.Tensor],
   keys = list(attributes.keys())
   parts = [_packed_attributes(attributes[k], framebuffer) for k in keys]
   widths = [p.shape[1] for p in parts]
-  cat = torch.cat(parts, dim=1) if len(parts) > 1 else parts[0]
+  cat = kernels.pack_columns(parts)
   bg = None
   if background_value is not None:
     bgv = torch.as_tensor(background_value, dtype=torch.float32, device=cat.device)

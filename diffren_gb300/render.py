@@ -54,7 +54,7 @@ def _render_fused(geom, attributes, shading_function, num_layers, face_culling_m
   widths = [p.shape[1] for p in parts]
   if sum(widths) > kernels._lib.DR_MAX_CHANNELS:
     return None
-  cat = torch.cat(parts, dim=1) if len(parts) > 1 else parts[0].contiguous()
+  cat = kernels.pack_columns(parts).contiguous()
   # Background samples are told by the depth buffer downstream, so their
   # ids and barycentrics need not be written; with a pass-through shader
   # (None) the splat is the only reader of the attributes, so neither are

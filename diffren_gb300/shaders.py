@@ -171,13 +171,23 @@ class _PointLight(torch.autograd.Function):
     if not any(need):
       return None, None, None, None, None
     d_out = d_out.float().contiguous()
-    grads = [torch.empty(ctx.n, 3, dtype=torch.float32, device=dif.device) if w else None
-             for w in need]
     sd, sn, sp = ctx.strides
+    # Inputs that are the columns of one packed buffer get their gradients as
+    # the columns of another, which the split's gradient then takes as it is.
+    start = min(t.storage_offset() for t in (dif, nrm, pos))
+    first = [t.storage_offset() - start for t in (dif, nrm, pos)]
+    if (all(need) and sd == sn == sp == 9 and sorted(first) == [0, 3, 6] and
+        len({t.untyped_storage().data_ptr() for t in (dif, nrm, pos)}) == 1):
+      packed = torch.empty(ctx.n, 9, dtype=torch.float32, device=dif.device)
+      grads, sg = [packed[:, f:f + 3] for f in first], 9
+    else:
+      grads = [torch.empty(ctx.n, 3, dtype=torch.float32, device=dif.device) if w else None
+               for w in need]
+      sg = 3
     with kernels._op("point_light_bwd", 1):
       rc = lib.dr_point_light_bwd(kernels._p(d_out), ctx.oc, kernels._p(dif), kernels._p(nrm),
                                   kernels._p(pos), ctx.n, sd, sn, sp, ctypes.byref(ctx.params),
-                                  *[kernels._p(g) for g in grads], 3,
+                                  *[kernels._p(g) for g in grads], sg,
                                   kernels._stream(dif.device))
     _lib.check(rc, "dr_point_light_bwd")
     return tuple(None if g is None else g.view(sh) for g, sh in zip(grads, ctx.shapes)) + (

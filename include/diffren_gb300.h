@@ -414,6 +414,17 @@ int dr_point_light_bwd(const float* d_out, int32_t out_channels, const float* di
                        float* d_diffuse, float* d_normals, float* d_positions,
                        int32_t grad_stride, void* stream);
 
+/* ------------------------------------------------- attribute columns */
+
+/* out [rows, K]: the columns of `count` parts side by side (K = the sum of
+ * widths, 1 <= count, K <= DR_MAX_CHANNELS), as jnp.concatenate along the
+ * last axis does for the attribute rows that the interpolation takes and in
+ * the gradient of splitting them again (interpolate.py:148-170). parts[i] is
+ * a device pointer to rows of widths[i] floats strides[i] floats apart, or
+ * null for zeros; the three arrays are host memory. */
+int dr_pack_columns(const float* const* parts, const int32_t* widths, const int64_t* strides,
+                    int32_t count, int64_t rows, float* out, void* stream);
+
 /* ------------------------------------------------------ compositing */
 
 /* CompositingMode.OVER of render_triangles (render.py:134-140): shaded

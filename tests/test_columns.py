@@ -1,0 +1,85 @@
+"""Packing attribute columns and splitting them again: values, gradients (also
+where the parts' gradients already share one buffer, or are missing) and
+forward mode, against torch.cat and torch.split."""
+import ctypes
+
+import pytest
+import torch
+
+from diffren_gb300 import _lib, kernels
+
+
+def test_pack_columns_rejects_bad_arguments():
+  lib = _lib.load()
+  one = (ctypes.c_int32 * 1)(3)
+  stride = (ctypes.c_int64 * 1)(3)
+  ptr = (ctypes.c_void_p * 1)(None)
+  for args in ((None, one, stride, 1, 4), (ptr, one, stride, 0, 4), (ptr, one, stride, 1, -1),
+               (ptr, (ctypes.c_int32 * 1)(17), stride, 1, 4), (ptr, one, stride, 1, 4)):
+    assert lib.dr_pack_columns(*args, None, None) == 1
+  two = (ctypes.c_int32 * 2)(9, 8)
+  assert lib.dr_pack_columns((ctypes.c_void_p * 2)(), two, (ctypes.c_int64 * 2)(9, 8), 2, 4, None,
+                             None) == 1
+  assert lib.dr_pack_columns(ptr, one, stride, 1, 0, None, None) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [0, 1, 127, 128, 129, 5000])
+@pytest.mark.parametrize("widths", [(3, 3, 3), (1, 1), (4, 12), (16,), (2, 5, 1, 7), (1,) * 16])
+def test_pack_and_split(rows, widths, device):
+  g = torch.Generator(device=device).manual_seed(rows)
+  wide = torch.randn(rows, 20, generator=g, device=device)
+  parts = [torch.randn(rows, w, generator=g, device=device).requires_grad_() for w in widths]
+  strided = [wide[:, i:i + w] for i, w in enumerate(widths) if i + w <= 20]
+  packed = kernels.pack_columns(parts)
+  assert torch.equal(packed, torch.cat(parts, 1))
+  if len(strided) == len(widths):
+    assert torch.equal(kernels._pack(strided, list(widths), rows, device), torch.cat(strided, 1))
+  split = kernels.split_channels(packed, list(widths))
+  for a, b in zip(split, torch.split(packed, list(widths), 1)):
+    assert torch.equal(a, b)
+  seeds = [torch.randn(rows, w, generator=g, device=device) for w in widths]
+  whole = torch.randn(rows, sum(widths), generator=g, device=device)
+  for grads in (seeds, torch.split(whole, list(widths), 1)):
+    used = list(range(0, len(widths), 2))  # every other part unused: no gradient
+    for which in (list(range(len(widths))), used):
+      got = torch.autograd.grad([split[i] for i in which], parts, [grads[i] for i in which],
+                                retain_graph=True, allow_unused=True)
+      for i, x in enumerate(got):
+        assert torch.equal(x, grads[i] if i in which else torch.zeros_like(grads[i]))
+
+
+@pytest.mark.gpu
+def test_pack_and_split_forward_mode(device):
+  import torch.autograd.forward_ad as fwAD
+  a, b = torch.randn(50, 3, device=device), torch.randn(50, 4, device=device)
+  da = torch.randn_like(a)
+  with fwAD.dual_level():
+    packed = kernels.pack_columns([fwAD.make_dual(a, da), b])
+    x, y = kernels.split_channels(packed, [3, 4])
+    assert torch.equal(fwAD.unpack_dual(x).tangent, da)
+    assert not fwAD.unpack_dual(y).tangent.any()
+
+
+# The columns of one [n, 9] buffer, in any order, get their gradients as the
+# columns of one buffer; the values are those of separate inputs.
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 3, 255, 256, 257, 1000])
+@pytest.mark.parametrize("order", [(0, 1, 2), (2, 0, 1)])
+@pytest.mark.parametrize("alpha", [False, True])
+def test_point_light_packed_gradients(rows, order, alpha, device):
+  from diffren_gb300 import shaders
+  g = torch.Generator(device=device).manual_seed(rows)
+  packed = torch.randn(rows, 9, generator=g, device=device)
+  seed = torch.randn(rows, 4 if alpha else 3, generator=g, device=device)
+  results = []
+  for split in (True, False):
+    p = packed.clone().requires_grad_()
+    cols = kernels.split_channels(p, [3, 3, 3])
+    if not split:
+      cols = [c.contiguous() for c in cols]
+    c = [cols[i] for i in order]
+    out = shaders.point_light(c[0], c[1], c[2], (2.0, 2.0, 2.0), ks=0.4, ns=3.0, alpha=alpha)
+    results.append((out.detach(), *torch.autograd.grad(out, [p], seed)))
+  for a, b in zip(*results):
+    assert torch.equal(a, b)
