@@ -112,11 +112,98 @@ __global__ void __launch_bounds__(256) over_bwd_kernel(OverArgs a, Batch B) {
   }
 }
 
+// Four channels in 16-byte aligned buffers (RGBA): one load per layer sample
+// and one store, each layer read once; the same operations in the same order.
+template <int LT>
+__global__ void __launch_bounds__(256) over_fwd4_kernel(OverArgs a, Batch B) {
+  const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (q >= B.pix_prefix[B.n]) return;
+  const OverPixel px = over_pixel(B, a.L, q);
+  const int L = a.L;
+  float4 s[LT];
+  float fg[LT];
+#pragma unroll
+  for (int l = 0; l < LT; ++l)
+    if (l < L) {
+      const int64_t e = px.e0 + l * px.hw;
+      fg[l] = __ldg(a.z + e) != 1.0f ? 1.0f : 0.0f;
+      s[l] = __ldg(reinterpret_cast<const float4*>(a.shaded) + e);
+    }
+  float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+  for (int l = LT - 1; l >= 0; --l)
+    if (l < L) {
+      const float4 v = make_float4(__fmul_rn(s[l].x, fg[l]), __fmul_rn(s[l].y, fg[l]),
+                                   __fmul_rn(s[l].z, fg[l]), __fmul_rn(s[l].w, fg[l]));
+      const float keep = __fsub_rn(1.0f, v.w);
+      o = l == L - 1 ? v
+                     : make_float4(__fadd_rn(v.x, __fmul_rn(keep, o.x)),
+                                   __fadd_rn(v.y, __fmul_rn(keep, o.y)),
+                                   __fadd_rn(v.z, __fmul_rn(keep, o.z)),
+                                   __fadd_rn(v.w, __fmul_rn(keep, o.w)));
+    }
+  reinterpret_cast<float4*>(a.out)[px.o] = o;
+}
+
+template <int LT>
+__global__ void __launch_bounds__(256) over_bwd4_kernel(OverArgs a, Batch B) {
+  const int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (q >= B.pix_prefix[B.n]) return;
+  const OverPixel px = over_pixel(B, a.L, q);
+  const int L = a.L;
+  float s[LT][4], fg[LT], keep[LT];
+#pragma unroll
+  for (int l = 0; l < LT; ++l)
+    if (l < L) {
+      const int64_t e = px.e0 + l * px.hw;
+      fg[l] = __ldg(a.z + e) != 1.0f ? 1.0f : 0.0f;
+      const float4 v = __ldg(reinterpret_cast<const float4*>(a.shaded) + e);
+      s[l][0] = __fmul_rn(v.x, fg[l]);
+      s[l][1] = __fmul_rn(v.y, fg[l]);
+      s[l][2] = __fmul_rn(v.z, fg[l]);
+      s[l][3] = __fmul_rn(v.w, fg[l]);
+      keep[l] = __fsub_rn(1.0f, s[l][3]);
+    }
+  // s[l] becomes the composite of the layers from l on.
+#pragma unroll
+  for (int l = LT - 2; l >= 0; --l)
+    if (l < L - 1)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        s[l][c] = __fadd_rn(s[l][c], __fmul_rn(keep[l], s[l + 1][c]));
+  const float4 d = __ldg(reinterpret_cast<const float4*>(a.d_out) + px.o);
+  float g[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+  for (int l = 0; l < LT; ++l)
+    if (l < L) {
+      float d_alpha = 0.0f;
+      if (l + 1 < L)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) d_alpha -= g[c] * s[l + 1 < LT ? l + 1 : l][c];
+      reinterpret_cast<float4*>(a.d_shaded)[px.e0 + l * px.hw] =
+          make_float4(g[0] * fg[l], g[1] * fg[l], g[2] * fg[l], (g[3] + d_alpha) * fg[l]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) g[c] = keep[l] * g[c];
+    }
+}
+
 template <int LT>
 void launch(const OverArgs& a, const Batch& b, bool backward, cudaStream_t stream) {
   const int64_t P = b.pix_prefix[b.n];
   if (P == 0) return;
   const unsigned blocks = unsigned((P + 255) / 256);
+  const uintptr_t all = reinterpret_cast<uintptr_t>(a.shaded) |
+                        reinterpret_cast<uintptr_t>(a.d_out) | reinterpret_cast<uintptr_t>(a.out) |
+                        reinterpret_cast<uintptr_t>(a.d_shaded);
+  if constexpr (LT <= 8) {
+    if (a.C == 4 && (all & 15) == 0) {
+      if (backward)
+        over_bwd4_kernel<LT><<<blocks, 256, 0, stream>>>(a, b);
+      else
+        over_fwd4_kernel<LT><<<blocks, 256, 0, stream>>>(a, b);
+      return;
+    }
+  }
   if (backward)
     over_bwd_kernel<LT><<<blocks, 256, 0, stream>>>(a, b);
   else
@@ -142,8 +229,13 @@ int over_launch(OverArgs a, const dr_image_desc* images, int n, bool backward,
   }
   for (int g0 = 0; g0 < n; g0 += DR_MAX_BATCH_INLINE) {
     make_batch(images + g0, std::min(n - g0, DR_MAX_BATCH_INLINE), a.L, 16, 16, b, err);
-    if (a.L <= 3)
-      launch<3>(a, b, backward, stream);
+    // The layers unroll to the next bound: registers for sixteen spill.
+    if (a.L <= 2)
+      launch<2>(a, b, backward, stream);
+    else if (a.L <= 4)
+      launch<4>(a, b, backward, stream);
+    else if (a.L <= 8)
+      launch<8>(a, b, backward, stream);
     else
       launch<DR_MAX_LAYERS>(a, b, backward, stream);
   }

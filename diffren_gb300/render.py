@@ -22,19 +22,64 @@ from . import rasterize
 from . import splat
 
 
+class _Slices(torch.autograd.Function):
+  """The slices of a tensor along its first dimension, as tensors over the
+  same memory. Their gradients come back as the buffer they share (what
+  stacking the shaded slices gives, when the shader returns its input) or
+  stacked in one pass, where a select per slice fills and adds a whole tensor
+  each. Plain tensors rather than views, so that a shader may still write to
+  its input; with several attributes (`views`) it may not, as with the views
+  of torch.split."""
+
+  @staticmethod
+  def forward(ctx, t, views):
+    ctx.shape, ctx.stride = t.shape, t.stride()
+    ctx.set_materialize_grads(False)
+    if views:
+      return t.unbind(0)
+    step = t.stride(0)
+    return tuple(
+        torch.empty(0, dtype=t.dtype, device=t.device).set_(
+            t.untyped_storage(), t.storage_offset() + i * step, t.shape[1:], t.stride()[1:])
+        for i in range(t.shape[0]))
+
+  @staticmethod
+  def jvp(ctx, d, _):
+    return tuple(d.unbind(0))
+
+  @staticmethod
+  def backward(ctx, *grads):
+    like = next((g for g in grads if g is not None), None)
+    if like is None:
+      return None, None
+    if all(g is not None and g.is_contiguous() for g in grads):
+      n = like.numel()
+      whole = kernels._one_buffer(grads, ctx.shape, (n, *like.stride()),
+                                  [i * n for i in range(len(grads))])
+      if whole is not None:
+        return whole, None
+    return torch.stack([torch.zeros_like(like) if g is None else g for g in grads]), None
+
+
 def _shade_layers(shading_function, interpolated, num_layers, batched):
   """vmap(shading_function) over layers (and images), as render.py:128."""
-  outs = []
-  if batched:
-    B = next(iter(interpolated.values())).shape[0]
-    for b in range(B):
-      outs.append(torch.stack([
-          shading_function({k: v[b, l] for k, v in interpolated.items()})
-          for l in range(num_layers)]))
-    return torch.stack(outs)
-  return torch.stack([
-      shading_function({k: v[l] for k, v in interpolated.items()})
-      for l in range(num_layers)])
+  first = next(iter(interpolated.values()))
+  lead = first.shape[:2] if batched else first.shape[:1]
+  n = lead.numel()
+  slices = {}
+  for k, v in interpolated.items():
+    flat = v.flatten(0, 1) if batched else v
+    if torch.is_grad_enabled() and v.requires_grad:
+      slices[k] = _Slices.apply(flat, len(interpolated) > 1)
+    else:
+      slices[k] = [flat[i] for i in range(n)]
+  outs = [shading_function({k: v[i] for k, v in slices.items()}) for i in range(n)]
+  if outs and not torch.is_grad_enabled():
+    for k, v in slices.items():
+      if all(o is s for o, s in zip(outs, v)):
+        return interpolated[k]  # the shader returned its input: nothing to stack
+  shaded = torch.stack(outs)
+  return shaded.view(*lead, *shaded.shape[1:]) if batched else shaded
 
 
 def _render_fused(geom, attributes, shading_function, num_layers, face_culling_mode,
