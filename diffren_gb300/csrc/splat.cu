@@ -560,6 +560,10 @@ __device__ __forceinline__ bool saved_wide(const SplatArgs& a) {
   return C == 4 && (reinterpret_cast<uintptr_t>(a.saved) & 15) == 0;
 }
 
+// Two and three layers save their taps' surface indexes (-2..2 in 3 bits).
+template <int LT>
+constexpr bool kCodes = LT == 2 || LT == 3;
+
 // A block covers a kTX x kTY tile of pixels, one per thread; the samples it
 // reads are the tile plus a 1-pixel halo: kRS x (kTY + 2) per layer.
 constexpr int kRS = kTX + 2;
@@ -872,7 +876,7 @@ __device__ __forceinline__ void splat_fwd_tile(const SplatArgs& a, const Batch& 
 
   float acc[3][4 * Q];
   float wacc[3] = {0.0f, 0.0f, 0.0f};
-  unsigned code = 0;  // surface codes of the 9 taps (three layers only)
+  unsigned code = 0;  // surface codes of the 9 taps (two and three layers)
   if (layers == 0) {
 #pragma unroll
     for (int k = 0; k < 3; ++k)
@@ -918,7 +922,7 @@ __device__ __forceinline__ void splat_fwd_tile(const SplatArgs& a, const Batch& 
         const float gap = fabsf(__fsub_rn(zS, zD)), deep = fabsf(__fsub_rn(1.0f, zS));
         const float minc = far < gap ? far : gap, mint = deep < gap ? deep : gap;
         const bool behind = mint < minc, front = !behind && far < gap;
-        if (LT == 3) code |= (behind ? 1u : front ? 3u : 2u) << (3 * j);
+        if (kCodes<LT>) code |= (behind ? 1u : front ? 3u : 2u) << (3 * j);
         const float w = __fmul_rn(wx[(u + 1) * kRR + s], wy[(v + 1) * kRR + s]);
         float4 c[Q];
 #pragma unroll
@@ -939,9 +943,9 @@ __device__ __forceinline__ void splat_fwd_tile(const SplatArgs& a, const Batch& 
         // start at a zero (or NaN) difference that no layer beats.
         if (tap[j])
           tap[j] |= unsigned((j == 4 ? 0 : surface_index(zs, s, p, L)) + 16) << 16;
-        // Surface index + 2 in 3 bits per tap (three layers: -2..2) for the
+        // Surface index + 2 in 3 bits per tap (up to three layers: -2..2) for the
         // VJP, which then needs no depths.
-        if (LT == 3 && tap[j]) code |= ((tap[j] >> 16) - 14u) << (3 * j);
+        if (kCodes<LT> && tap[j]) code |= ((tap[j] >> 16) - 14u) << (3 * j);
       }
       for (int l = 0; l < L; ++l) {
         if (!((layers >> l) & 1u)) continue;
@@ -1007,7 +1011,7 @@ __device__ __forceinline__ void splat_fwd_tile(const SplatArgs& a, const Batch& 
         for (int c = 0; c < C; ++c) a.saved[(k * (C + 1) + c) * a.P + pix] = acc[k][c];
         a.saved[(k * (C + 1) + C) * a.P + pix] = wacc[k];
       }
-      if (LT == 3) reinterpret_cast<unsigned*>(a.saved)[3 * (C + 1) * a.P + pix] = code;
+      if (kCodes<LT>) reinterpret_cast<unsigned*>(a.saved)[3 * (C + 1) * a.P + pix] = code;
     }
   }
   if (a.accum || a.normalized) {
@@ -1234,17 +1238,19 @@ __device__ __forceinline__ void splat_bwd_tile(const SplatArgs& a, const Batch& 
           for (int c = 0; c < C; ++c) acc[k][c] = __ldg(a.saved + (k * (C + 1) + c) * a.P + pix);
           wacc[k] = __ldg(a.saved + (k * (C + 1) + C) * a.P + pix);
         }
-        if (LT == 3 && a.zb)
+        if (kCodes<LT> && a.zb)
           code = __ldg(reinterpret_cast<const unsigned*>(a.saved) + 3 * (C + 1) * a.P + pix);
       }
       float d[C];
       load_row<C>(a.d_out + pix * C, d);
       accum_adjoint<C>(acc, wacc, d, g, h);
       const int64_t eq = lbase + int64_t(qy) * W + qx;
-      if (LT == 3 && a.zb) {
+      if (kCodes<LT> && a.zb) {
         // The forward's surface codes of this pixel's taps replace the
         // depths (the zs area holds them).
         reinterpret_cast<unsigned*>(zs)[i] = code;
+      } else if (LT == 1) {
+        // one layer: every tap is at the surface, no depth is compared
       } else if (a.zb) {
         unsigned m = 0;
         for (int l = 0; l < L; ++l) m |= unsigned(__ldg(a.zb + eq + l * HW) != 1.0f) << l;
@@ -1290,7 +1296,7 @@ __device__ __forceinline__ void splat_bwd_tile(const SplatArgs& a, const Batch& 
       const int px = sx + u, py = sy + v;
       const bool in = mine && px >= 0 && py >= 0 && px < W && py < H;
       ok |= unsigned(in) << j;
-      if (LT == 3)  // pixel s1 + (u, v) saw this sample as its tap j
+      if (kCodes<LT>)  // pixel s1 + (u, v) saw this sample as its tap j
         surf[j] = in ? int((reinterpret_cast<const unsigned*>(zs)[s1 + v * kRS + u] >>
                             (3 * j)) & 7u) - 2
                      : 0;
@@ -1394,7 +1400,7 @@ __device__ __forceinline__ void splat_bwd_tile(const SplatArgs& a, const Batch& 
 }
 
 template <int C, int LT>
-__global__ void __launch_bounds__(256, (C <= 4 && LT == 3) ? 5 : 4)
+__global__ void __launch_bounds__(256, (C <= 4 && LT > 0) ? 5 : 4)
     splat_bwd_kernel(SplatArgs a, Batch B) {
   extern __shared__ __align__(16) float smem[];
   splat_bwd_tile<C, LT>(a, B, blockIdx.x, smem);
@@ -1403,7 +1409,7 @@ __global__ void __launch_bounds__(256, (C <= 4 && LT == 3) ? 5 : 4)
 // Persistent blocks over the tiles the forward listed, handed out by the
 // backward's work counter (reset by splat_bwd_zero_kernel, which runs first).
 template <int C, int LT>
-__global__ void __launch_bounds__(256, (C <= 4 && LT == 3) ? 5 : 4)
+__global__ void __launch_bounds__(256, (C <= 4 && LT > 0) ? 5 : 4)
     splat_bwd_list_kernel(SplatArgs a, Batch B, TileList t) {
   extern __shared__ __align__(16) float smem[];
   __shared__ int s_item;
@@ -1693,6 +1699,7 @@ int run_splat_jvp(const SplatArgs& a, const float4* d_vp, const float* d_colors,
 int dispatch(bool bwd, int C, const SplatArgs& a, const dr_image_desc* images, int n,
              cudaStream_t stream, std::string& err) {
   if (C == 4 && a.L == 3) return run_splat<4, 3>(bwd, a, images, n, stream, err);
+  if (C == 4 && a.L == 2) return run_splat<4, 2>(bwd, a, images, n, stream, err);
   if (C == 4 && a.L == 1) return run_splat<4, 1>(bwd, a, images, n, stream, err);
   switch (C) {
     case 1: return run_splat<1, 0>(bwd, a, images, n, stream, err);
