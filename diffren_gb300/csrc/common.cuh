@@ -254,6 +254,22 @@ __device__ __forceinline__ bool fits_fixed32(float4 v0, float4 v1, float4 v2) {
          fabsf(v2.w) < lim;
 }
 
+// The coefficients of coordinates that do not fit 32 bits.
+static __device__ __noinline__ void edge_matrix_wide(float4 v0, float4 v1, float4 v2, long long* m) {
+  const long long y0 = to_fixed(v0.y), y1 = to_fixed(v1.y), y2 = to_fixed(v2.y);
+  const long long w0 = to_fixed(v0.w), w1 = to_fixed(v1.w), w2 = to_fixed(v2.w);
+  const long long x0 = to_fixed(v0.x), x1 = to_fixed(v1.x), x2 = to_fixed(v2.x);
+  m[0] = wsub(wmul(y1, w2), wmul(w1, y2));
+  m[1] = wsub(wmul(x2, w1), wmul(w2, x1));
+  m[2] = wsub(wmul(x1, y2), wmul(y1, x2));
+  m[3] = wsub(wmul(y2, w0), wmul(w2, y0));
+  m[4] = wsub(wmul(x0, w2), wmul(w0, x2));
+  m[5] = wsub(wmul(x2, y0), wmul(y2, x0));
+  m[6] = wsub(wmul(y0, w1), wmul(w0, y1));
+  m[7] = wsub(wmul(x1, w0), wmul(w1, x0));
+  m[8] = wsub(wmul(x0, y1), wmul(y0, x1));
+}
+
 // ComputeUnnormalizedMatrixInverse (rasterize_utils.h:176-206) of the matrix
 // with columns (x_i, y_i, w_i) in 16.16 fixed point. Row i of m holds the
 // coefficients (a, b, c) of edge function i. For NONE and FRONT the reference
@@ -282,18 +298,11 @@ __device__ __forceinline__ void edge_matrix(float4 v0, float4 v1, float4 v2, int
     m[8] = det2(a0, y1, y0, a1);
     x0 = a0; x1 = a1; x2 = a2;
   } else {
-    const long long y0 = to_fixed(v0.y), y1 = to_fixed(v1.y), y2 = to_fixed(v2.y);
-    const long long w0 = to_fixed(v0.w), w1 = to_fixed(v1.w), w2 = to_fixed(v2.w);
+    long long t[9];
+    edge_matrix_wide(v0, v1, v2, t);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) m[i] = t[i];
     x0 = to_fixed(v0.x); x1 = to_fixed(v1.x); x2 = to_fixed(v2.x);
-    m[0] = wsub(wmul(y1, w2), wmul(w1, y2));
-    m[1] = wsub(wmul(x2, w1), wmul(w2, x1));
-    m[2] = wsub(wmul(x1, y2), wmul(y1, x2));
-    m[3] = wsub(wmul(y2, w0), wmul(w2, y0));
-    m[4] = wsub(wmul(x0, w2), wmul(w0, x2));
-    m[5] = wsub(wmul(x2, y0), wmul(y2, x0));
-    m[6] = wsub(wmul(y0, w1), wmul(w0, y1));
-    m[7] = wsub(wmul(x1, w0), wmul(w1, x0));
-    m[8] = wsub(wmul(x0, y1), wmul(y0, x1));
   }
   if (culling == DR_CULL_NONE || culling == DR_CULL_FRONT) {
     const long long det_i = wadd(wadd(wmul(x0, m[0]), wmul(x1, m[3])), wmul(x2, m[6]));
@@ -397,29 +406,10 @@ __device__ __forceinline__ uint64_t shift_round_even(uint64_t x, int s) {
   return q + ((rem > half || (rem == half && (q & 1))) ? 1 : 0);
 }
 
-// Exact integer form of discretize_z_fp64 for z in [-1, 1] or NaN:
-// a = RN_double(z + 1) as N * 2^-sh, then floor(RN_double(a * S)).
-__device__ __forceinline__ uint32_t discretize_z(float z) {
-  const uint32_t bits = __float_as_uint(z);
-  const uint32_t mag = bits & 0x7fffffffu;
-  // NaN: (NaN + 1) * S converts to 0x80000000 on the GPU (checked against
-  // discretize_z_fp64 by dr_selftest_depth_codec). A constant keeps the
-  // double-precision path out of the rasterizer entirely.
-  if (mag > 0x7f800000u) return 0x80000000u;
-  if (mag == 0) return 2147483647u;  // (0 + 1) * S
-  const bool neg = bits >> 31;
-  const int bexp = int(mag >> 23);
-  if (bexp >= 120 && bexp <= 126) {
-    // 2^-7 <= |z| < 1 (every visible depth but those near 0): the same
-    // computation as below with sh = 24..30, where N < 2^31 and P < 2^62
-    // fit 32- and 64-bit integers.
-    const int sh = 150 - bexp;
-    const uint32_t m = (mag & 0x7fffffu) | 0x800000u;
-    const uint32_t n = neg ? (1u << sh) - m : (1u << sh) + m;
-    const uint64_t P = uint64_t(n) * 2147483647u;
-    const uint64_t frac_mask = (1ull << sh) - 1;
-    if ((P & frac_mask) < frac_mask + 1 - (1ull << (sh - 22))) return uint32_t(P >> sh);
-  }
+// The rest of discretize_z. Out of line, like the other rare paths here (two
+// such codecs and the 64-bit edge matrix inlined made the fine kernel miss the
+// instruction cache: 338 -> 323 us on the 8 x 1024^2 sphere without them).
+static __device__ __noinline__ uint32_t discretize_z_general(uint32_t mag, int bexp, bool neg) {
   const uint64_t M = bexp ? ((mag & 0x7fffffu) | 0x800000u) : (mag & 0x7fffffu);
   const int E = bexp ? bexp - 150 : -149;  // |z| = M * 2^E
   uint64_t N;
@@ -449,29 +439,35 @@ __device__ __forceinline__ uint32_t discretize_z(float z) {
   return uint32_t(Q >> sh);
 }
 
-// Exact integer form of undiscretize_z_fp64: q = RN_double(d / S) from the
-// repeating base-2^31 expansion of d / S, r = RN_double(q - 1), then
-// RN_float(r). Fixed point in units of 2^-83 (q >= 1/S has ulp >= 2^-83).
-__device__ __forceinline__ float undiscretize_z(uint32_t d) {
-  const uint32_t S = 2147483647u;
-  if (d >= S && d < 2 * S) {
-    // q = d / S in [1, 2) (every depth in [0, 1)): with e = d - S and
-    // T = e (2^31 + 1), floor(e / S * 2^93) / 2^41 = e 2^21 + T / 2^41, so
-    // RN_double(q) - 1 = R 2^-52 with R = e 2^21 + T >> 41 + bit 40 of T
-    // (the remainder is never zero, so there are no ties), exact in double;
-    // then R rounds to 24 bits, ties to even.
-    const uint64_t e = d - S;
-    const uint64_t T = (e << 31) + e;
-    const uint64_t R = (e << 21) + (T >> 41) + ((T >> 40) & 1u);
-    if (R == 0) return 0.0f;
-    const int bl = 64 - __clzll(R);
-    if (bl <= 24) return float(uint32_t(R)) * 0x1p-52f;
-    const int g = bl - 24;
-    uint64_t mant = R >> g;
-    const uint64_t rem = R & ((1ull << g) - 1), half = 1ull << (g - 1);
-    if (rem > half || (rem == half && (mant & 1))) ++mant;
-    return float(uint32_t(mant)) * __uint_as_float(uint32_t(127 + g - 52) << 23);
+// Exact integer form of discretize_z_fp64 for z in [-1, 1] or NaN:
+// a = RN_double(z + 1) as N * 2^-sh, then floor(RN_double(a * S)).
+__device__ __forceinline__ uint32_t discretize_z(float z) {
+  const uint32_t bits = __float_as_uint(z);
+  const uint32_t mag = bits & 0x7fffffffu;
+  // NaN: (NaN + 1) * S converts to 0x80000000 on the GPU (checked against
+  // discretize_z_fp64 by dr_selftest_depth_codec). A constant keeps the
+  // double-precision path out of the rasterizer entirely.
+  if (mag > 0x7f800000u) return 0x80000000u;
+  if (mag == 0) return 2147483647u;  // (0 + 1) * S
+  const bool neg = bits >> 31;
+  const int bexp = int(mag >> 23);
+  if (bexp >= 120 && bexp <= 126) {
+    // 2^-7 <= |z| < 1 (every visible depth but those near 0): the same
+    // computation as below with sh = 24..30, where N < 2^31 and P < 2^62
+    // fit 32- and 64-bit integers.
+    const int sh = 150 - bexp;
+    const uint32_t m = (mag & 0x7fffffu) | 0x800000u;
+    const uint32_t n = neg ? (1u << sh) - m : (1u << sh) + m;
+    const uint64_t P = uint64_t(n) * 2147483647u;
+    const uint64_t frac_mask = (1ull << sh) - 1;
+    if ((P & frac_mask) < frac_mask + 1 - (1ull << (sh - 22))) return uint32_t(P >> sh);
   }
+  return discretize_z_general(mag, bexp, neg);
+}
+
+// The rest of undiscretize_z.
+static __device__ __noinline__ float undiscretize_z_general(uint32_t d) {
+  const uint32_t S = 2147483647u;
   const u128 one = 1;
   const uint32_t I = (d >= S) + (d >= 2 * S);
   const uint64_t e = d - uint64_t(I) * S;  // d / S = I + e / S, e < S
@@ -516,6 +512,32 @@ __device__ __forceinline__ float undiscretize_z(uint32_t d) {
   const float mant = float(uint32_t(R >> g));  // exact (< 2^24)
   const float v = ldexpf(mant, g - 83);
   return rneg ? -v : v;
+}
+
+// Exact integer form of undiscretize_z_fp64: q = RN_double(d / S) from the
+// repeating base-2^31 expansion of d / S, r = RN_double(q - 1), then
+// RN_float(r). Fixed point in units of 2^-83 (q >= 1/S has ulp >= 2^-83).
+__device__ __forceinline__ float undiscretize_z(uint32_t d) {
+  const uint32_t S = 2147483647u;
+  if (d >= S && d < 2 * S) {
+    // q = d / S in [1, 2) (every depth in [0, 1)): with e = d - S and
+    // T = e (2^31 + 1), floor(e / S * 2^93) / 2^41 = e 2^21 + T / 2^41, so
+    // RN_double(q) - 1 = R 2^-52 with R = e 2^21 + T >> 41 + bit 40 of T
+    // (the remainder is never zero, so there are no ties), exact in double;
+    // then R rounds to 24 bits, ties to even.
+    const uint64_t e = d - S;
+    const uint64_t T = (e << 31) + e;
+    const uint64_t R = (e << 21) + (T >> 41) + ((T >> 40) & 1u);
+    if (R == 0) return 0.0f;
+    const int bl = 64 - __clzll(R);
+    if (bl <= 24) return float(uint32_t(R)) * 0x1p-52f;
+    const int g = bl - 24;
+    uint64_t mant = R >> g;
+    const uint64_t rem = R & ((1ull << g) - 1), half = 1ull << (g - 1);
+    if (rem > half || (rem == half && (mant & 1))) ++mant;
+    return float(uint32_t(mant)) * __uint_as_float(uint32_t(127 + g - 52) << 23);
+  }
+  return undiscretize_z_general(d);
 }
 
 // Order-preserving float -> uint32 map with -0 == +0 (float depth keys).
