@@ -61,14 +61,16 @@ constexpr int kMaxDevices = 64;
 
 // Host-side cache of one kernel's launch attributes on each device: the
 // dynamic shared-memory limit raised so far, and SMs x resident blocks per
-// SM for one shared-memory size. Host threads may launch concurrently, so
-// every use holds the lock; the limit only grows.
+// SM for the last few shared-memory sizes. Host threads may launch
+// concurrently, so every use holds the lock; the limit only grows.
 struct LaunchCache {
+  static constexpr int kSizes = 4;
   std::mutex mu;
   size_t raised[kMaxDevices] = {};
-  size_t occ_smem[kMaxDevices] = {};
+  size_t occ_smem[kMaxDevices][kSizes] = {};
+  int per_sm[kMaxDevices][kSizes] = {};  // 0: free
   int sms[kMaxDevices] = {};
-  int per_sm[kMaxDevices] = {};
+  int next[kMaxDevices] = {};
 };
 
 // Raises kern's dynamic shared-memory limit on the current device to smem
@@ -92,16 +94,20 @@ bool prepare_launch(LaunchCache& c, K kern, int threads, size_t smem, int& sms, 
     }
     c.raised[dev] = smem;
   }
-  if (c.per_sm[dev] == 0 || c.occ_smem[dev] != smem) {
-    int n = 0, p = 0;
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, kern, threads, smem);
-    c.sms[dev] = std::max(1, n);
-    c.per_sm[dev] = std::max(1, p);
-    c.occ_smem[dev] = smem;
-  }
-  sms = c.sms[dev];
-  per_sm = c.per_sm[dev];
+  for (int k = 0; k < LaunchCache::kSizes; ++k)
+    if (c.per_sm[dev][k] != 0 && c.occ_smem[dev][k] == smem) {
+      sms = c.sms[dev];
+      per_sm = c.per_sm[dev][k];
+      return true;
+    }
+  int n = 0, p = 0;
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, kern, threads, smem);
+  const int k = c.next[dev];
+  c.next[dev] = (k + 1) % LaunchCache::kSizes;
+  sms = c.sms[dev] = std::max(1, n);
+  per_sm = c.per_sm[dev][k] = std::max(1, p);
+  c.occ_smem[dev][k] = smem;
   return true;
 }
 

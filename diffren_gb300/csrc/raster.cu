@@ -9,6 +9,7 @@
 // pixel keeps the L smallest packed (depth | triangle id) keys, which is
 // independent of the order fragments arrive in.
 #include <algorithm>
+#include <cstdint>
 #include <cstring>
 #include <string>
 
@@ -990,7 +991,7 @@ bool check_config(const dr_raster_config* cfg, int& L, int& TW, int& TH, int& la
   if (!cfg) { err = "config is null"; return false; }
   L = cfg->num_layers;
   TW = resolve_tile(cfg->tile_width);
-  TH = resolve_tile(cfg->tile_height);
+  TH = resolve_tile(cfg->tile_height);  // see group_batch where neither is given
   large = cfg->large_tiles > 0 ? cfg->large_tiles : kDefaultLargeTiles;
   if (L < 1 || L > DR_MAX_LAYERS) { err = "num_layers must be in [1, 16]"; return false; }
   if (cfg->face_culling_mode < 0 || cfg->face_culling_mode > 2) {
@@ -1009,6 +1010,58 @@ bool check_config(const dr_raster_config* cfg, int& L, int& TW, int& TH, int& la
     err = "unknown raster config flags";
     return false;
   }
+  return true;
+}
+
+// Tile of a group of images whose configuration gives none, from its 16x16
+// tiles and its triangles. Few tiles leave most of the 1216 resident blocks
+// idle, and where there are triangles enough smaller tiles spread them: setup
+// to fine kernel for a 100k-triangle sphere takes 57 us at 256x256 with 8x8
+// tiles, 90 with 16x16; at 768x768 61 with 16x8, 83 with 16x16; from 8192 tiles
+// on 16x16 is the best (122 us, 129 with 16x8), and with fewer than 16
+// triangles a tile already above 512 (5000 triangles at 768x768: 45, 53 us).
+// The threshold of the large list stays at the same number of pixels. Many
+// tiles with few triangles each are bound by the cost per tile: the 64-mesh ragged batch (111k tiles)
+// takes 1075 us with 32x16, 1183 with 16x16; with more than 24 triangles a
+// tile they are equal (terrain 778, 766), and above four layers the keys of
+// a 32x16 tile cost more blocks per SM than it gains (eight: 1788, 1752).
+void default_tile(int64_t tiles16, int64_t tris, int L, int& TW, int& TH) {
+  TW = TH = kDefaultTile;
+  if (tiles16 <= 512 || (tiles16 <= 1536 && tris >= 16 * tiles16)) {
+    TW = TH = 8;
+  } else if (tiles16 <= 6144 && tris >= 16 * tiles16) {
+    TH = 8;
+  } else if (tiles16 >= 16384 && L <= 4 && tris <= 24 * tiles16) {
+    TW = 32;
+  }
+}
+
+// The batch table of one group with its tiles, and the workspace it needs.
+// With a tile by the rule that workspace may exceed the 16x16 one, which is
+// then enough too (at 16x16): `min_bytes` is what a call must bring.
+bool group_batch(const dr_image_desc* images, int n, const dr_raster_config* cfg, int L,
+                 size_t ws_bytes, int& TW, int& TH, int& large, Batch& b, Layout& lay,
+                 size_t& min_bytes, std::string& err) {
+  if (!make_batch(images, n, L, TW, TH, b, err)) return false;
+  lay = make_layout(b.tri_start[n], b.tile_start[n], n, large);
+  min_bytes = lay.total;
+  if (cfg->tile_width > 0 || cfg->tile_height > 0) return true;
+  int w, h;
+  default_tile(b.tile_start[n], b.tri_start[n], L, w, h);
+  if (w == TW && h == TH) return true;
+  Batch ruled;
+  std::string ignored;
+  if (!make_batch(images, n, L, w, h, ruled, ignored)) return true;  // too many tiles
+  int ruled_large = large;
+  if (cfg->large_tiles <= 0)
+    ruled_large = std::max(large, large * kDefaultTile * kDefaultTile / (w * h));
+  const Layout l = make_layout(ruled.tri_start[n], ruled.tile_start[n], n, ruled_large);
+  if (l.total > ws_bytes) return true;
+  b = ruled;
+  lay = l;
+  large = ruled_large;
+  TW = w;
+  TH = h;
   return true;
 }
 
@@ -1032,9 +1085,12 @@ size_t raster_workspace_bytes(const dr_image_desc* images, int n,
   for (int g0 = 0; g0 < n; g0 += DR_MAX_BATCH_INLINE) {
     const int cnt = std::min(n - g0, DR_MAX_BATCH_INLINE);
     Batch b;
-    if (!make_batch(images + g0, cnt, L, TW, TH, b, err)) return 0;
-    const Layout lay = make_layout(b.tri_start[cnt], b.tile_start[cnt], cnt, large);
-    best = std::max(best, lay.total);
+    Layout lay;
+    int w = TW, h = TH, tiles = large;
+    size_t min_bytes;
+    if (!group_batch(images + g0, cnt, cfg, L, SIZE_MAX, w, h, tiles, b, lay, min_bytes, err))
+      return 0;
+    best = std::max(best, std::max(min_bytes, lay.total));
   }
   return best;
 }
@@ -1075,7 +1131,6 @@ int raster_launch(const float* vertices, const int32_t* triangles,
       return DR_ERR_MISALIGNED;
     }
   }
-  const size_t smem = fine_smem_bytes(L, TW, TH);
   const bool fused = so.positions != nullptr;
   // Instantiations: fused or not, three layers or any.
   using Fine = void (*)(RasterArgs, Batch);
@@ -1085,20 +1140,26 @@ int raster_launch(const float* vertices, const int32_t* triangles,
                         fine_raster_kernel<true, 0>, fine_raster_kernel<true, 3>};
   const Prep prep[4] = {prepare_fine<false, 0>, prepare_fine<false, 3>,
                         prepare_fine<true, 0>, prepare_fine<true, 3>};
-  int sms = 0, per_sm = 0;
-  if (!prep[variant](smem, sms, per_sm, err)) return DR_ERR_INVALID_ARGUMENT;
-
+  const int TW0 = TW, TH0 = TH, large0 = large;
   for (int g0 = 0; g0 < n; g0 += DR_MAX_BATCH_INLINE) {
     const int cnt = std::min(n - g0, DR_MAX_BATCH_INLINE);
     Batch b;
-    if (!make_batch(images + g0, cnt, L, TW, TH, b, err)) return DR_ERR_INVALID_ARGUMENT;
+    Layout lay;
+    size_t min_bytes;
+    TW = TW0;
+    TH = TH0;
+    large = large0;
+    if (!group_batch(images + g0, cnt, cfg, L, ws_bytes, TW, TH, large, b, lay, min_bytes, err))
+      return DR_ERR_INVALID_ARGUMENT;
     const int64_t tris = b.tri_start[cnt];
     const int tiles = b.tile_start[cnt];
-    const Layout lay = make_layout(tris, tiles, cnt, large);
-    if (lay.total > ws_bytes) {
-      err = "workspace too small: need " + std::to_string(lay.total) + " bytes";
+    if (min_bytes > ws_bytes) {
+      err = "workspace too small: need " + std::to_string(min_bytes) + " bytes";
       return DR_ERR_WORKSPACE_TOO_SMALL;
     }
+    const size_t smem = fine_smem_bytes(L, TW, TH);
+    int sms = 0, per_sm = 0;
+    if (!prep[variant](smem, sms, per_sm, err)) return DR_ERR_INVALID_ARGUMENT;
     char* ws = static_cast<char*>(workspace);
     RasterArgs a;
     a.verts = reinterpret_cast<const float4*>(vertices);

@@ -128,8 +128,8 @@ extern "C" int dr_rasterize_triangles_static_scratch(
   c.num_layers = num_layers;
   c.face_culling_mode = face_culling_mode;
   c.depth_mode = depth_mode;
-  c.tile_width = 0;
-  c.tile_height = 0;
+  c.tile_width = 16;  // a fixed tile: what the fixed scratch admits does not
+  c.tile_height = 16;  // move with the rule for the default one
   c.large_tiles = 0;
   c.flags = 0;
   // Size check first: nothing runs on the GPU for an oversized request.

@@ -99,8 +99,9 @@ typedef struct dr_raster_config {
   int32_t num_layers;        /* L >= 1, at most DR_MAX_LAYERS */
   int32_t face_culling_mode; /* DR_CULL_* */
   int32_t depth_mode;        /* DR_DEPTH_* */
-  int32_t tile_width;        /* fine-raster tile, 0 = default (16) */
-  int32_t tile_height;       /* 0 = default (16); tile_width*tile_height <= 1024 */
+  int32_t tile_width;        /* fine-raster tile, 0 = default (16; with both
+                                0 by the batch's tiles and triangles) */
+  int32_t tile_height;       /* 0 = default; tile_width*tile_height <= 1024 */
   int32_t large_tiles;       /* triangles spanning more tiles than this go to a
                                 per-image list every tile scans; 0 = default */
   uint32_t flags;            /* DR_RASTER_* bits, 0 = none */

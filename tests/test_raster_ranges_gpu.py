@@ -1,6 +1,8 @@
 """GPU rasterizer against the oracle over the ranges its dispatch rules split:
 edge-function magnitudes, row alignments and channel counts of the background
-rows, layer counts."""
+rows, layer counts, the default tile."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -57,3 +59,40 @@ def test_background_and_layers_match_oracle(w, h, layers, channels, device):
     assert torch.equal(a, want)  # 0 on background
     fg = z != 1.0
     assert torch.equal(pos[fg][:, :3], want_pos[fg][:, :3])
+
+
+# The default tile follows the batch's 16x16 tiles (512, 1536, 2560, 6144,
+# 16384) and triangles per tile (16, 24): both sides of each line give the
+# bits of an explicit tile, and a workspace for 16x16 tiles is enough.
+@pytest.mark.parametrize("images,w,h,tris,layers", [
+    (1, 352, 360, 300, 3), (1, 352, 376, 300, 3), (1, 352, 376, 9000, 2), (6, 256, 256, 5000, 3),
+    (6, 256, 272, 5000, 3), (10, 256, 256, 200, 1), (11, 256, 256, 200, 4), (11, 256, 256, 4500, 3),
+    (24, 256, 256, 5000, 3), (64, 256, 256, 300, 3), (64, 250, 256, 300, 4), (64, 256, 256, 300, 5),
+    (64, 256, 256, 6200, 3), (130, 64, 48, 40, 3)])
+def test_default_tile_rule(images, w, h, tris, layers, device):
+  clips = []
+  for i in range(min(images, 3)):
+    verts, tri = _scene("soup", tris, w, h, i)
+    clips.append(torch.tensor(np.asarray(verts, np.float32), device=device))
+  v, t = len(clips[0]), len(tri)
+  clip = torch.cat([clips[i % len(clips)] for i in range(images)])
+  tri = torch.tensor(np.asarray(tri, np.int32), device=device).repeat(images, 1)
+  batch = kernels.ImageBatch([w] * images, [h] * images, [v] * images, [t] * images)
+  config = lambda tile: kernels.raster_config(layers, 1, _lib.DR_DEPTH_DISCRETIZED, tile)
+  want = kernels.rasterize_packed(clip, tri, batch, config((16, 16)))
+  got = kernels.rasterize_packed(clip, tri, batch, config((0, 0)))
+  for a, b in zip(got, want):
+    assert torch.equal(a, b)
+  need = kernels.raster_workspace_bytes(batch, config((16, 16)))
+  assert kernels.raster_workspace_bytes(batch, config((0, 0))) >= need
+  lib, P = _lib.load(), kernels._p
+  ws = torch.empty(need, dtype=torch.uint8, device=device)
+  for size, ok in ((need, True), (need - 256, False)):
+    out = [torch.full_like(x, -7) for x in want]
+    cfg = config((0, 0))
+    rc = lib.dr_rasterize_batch(P(clip), P(tri), batch.ptr, batch.n, ctypes.byref(cfg), P(out[0]),
+                                P(out[1]), P(out[2]), P(ws), size, kernels._stream(device))
+    assert (rc == 0) == ok
+    if ok:
+      for a, b in zip(out, want):
+        assert torch.equal(a, b)
