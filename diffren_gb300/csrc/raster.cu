@@ -1013,26 +1013,44 @@ bool check_config(const dr_raster_config* cfg, int& L, int& TW, int& TH, int& la
   return true;
 }
 
-// Tile of a group of images whose configuration gives none, from its 16x16
-// tiles and its triangles. Few tiles leave most of the 1216 resident blocks
-// idle, and where there are triangles enough smaller tiles spread them: setup
-// to fine kernel for a 100k-triangle sphere takes 57 us at 256x256 with 8x8
+// Tile of a group of images whose configuration gives none, from its table
+// with 16x16 tiles. Few tiles leave most of the 1216 resident blocks idle,
+// and where there are triangles enough smaller tiles spread them: setup to
+// fine kernel for a 100k-triangle sphere takes 57 us at 256x256 with 8x8
 // tiles, 90 with 16x16; at 768x768 61 with 16x8, 83 with 16x16; from 8192 tiles
 // on 16x16 is the best (122 us, 129 with 16x8), and with fewer than 16
 // triangles a tile already above 512 (5000 triangles at 768x768: 45, 53 us).
-// The threshold of the large list stays at the same number of pixels. Many
-// tiles with few triangles each are bound by the cost per tile: the 64-mesh ragged batch (111k tiles)
-// takes 1075 us with 32x16, 1183 with 16x16; with more than 24 triangles a
-// tile they are equal (terrain 778, 766), and above four layers the keys of
-// a 32x16 tile cost more blocks per SM than it gains (eight: 1788, 1752).
-void default_tile(int64_t tiles16, int64_t tris, int L, int& TW, int& TH) {
+// The threshold of the large list stays at the same number of pixels.
+// Many tiles with few triangles each are bound by the cost per tile: the
+// 64-mesh ragged batch (111k tiles) takes 1069 us with 32x16, 1174 with 16x16;
+// with more than 24 triangles a tile they are equal (terrain 770, 762). An
+// image whose tiles hold more than their share of all the triangles (of 912
+// resident blocks) then sets the time: one with 1531 a tile among 979k took
+// 595 us with 32x16, 518 with 16x16. Above four layers the keys of a 32x16
+// tile cost more blocks per SM than it gains (eight: 1788, 1752). Rows that do
+// not start on 32 bytes leave partial sectors at both ends, half as many with
+// tiles twice as wide (terrain at 2047 pixels: 841 with 32x8, 878).
+void default_tile(const Batch& b, int L, int& TW, int& TH) {
+  const int64_t tiles = b.tile_start[b.n], tris = b.tri_start[b.n];
   TW = TH = kDefaultTile;
-  if (tiles16 <= 512 || (tiles16 <= 1536 && tris >= 16 * tiles16)) {
+  if (tiles <= 512 || (tiles <= 1536 && tris >= 16 * tiles)) {
     TW = TH = 8;
-  } else if (tiles16 <= 6144 && tris >= 16 * tiles16) {
+  } else if (tiles <= 6144 && tris >= 16 * tiles) {
     TH = 8;
-  } else if (tiles16 >= 16384 && L <= 4 && tris <= 24 * tiles16) {
-    TW = 32;
+  } else if (tiles >= 16384) {
+    bool even = true;
+    int64_t unaligned = 0;
+    for (int i = 0; i < b.n; ++i) {
+      const int64_t t = b.tile_start[i + 1] - b.tile_start[i];
+      if (912 * (b.tri_start[i + 1] - b.tri_start[i]) > tris * t) even = false;
+      if (b.width[i] % 8 != 0) unaligned += t;
+    }
+    if (L <= 4 && tris <= 24 * tiles && even) {
+      TW = 32;
+    } else if (2 * unaligned > tiles) {
+      TW = 32;
+      TH = 8;
+    }
   }
 }
 
@@ -1047,7 +1065,7 @@ bool group_batch(const dr_image_desc* images, int n, const dr_raster_config* cfg
   min_bytes = lay.total;
   if (cfg->tile_width > 0 || cfg->tile_height > 0) return true;
   int w, h;
-  default_tile(b.tile_start[n], b.tri_start[n], L, w, h);
+  default_tile(b, L, w, h);
   if (w == TW && h == TH) return true;
   Batch ruled;
   std::string ignored;

@@ -61,14 +61,14 @@ def test_background_and_layers_match_oracle(w, h, layers, channels, device):
     assert torch.equal(pos[fg][:, :3], want_pos[fg][:, :3])
 
 
-# The default tile follows the batch's 16x16 tiles (512, 1536, 2560, 6144,
-# 16384) and triangles per tile (16, 24): both sides of each line give the
-# bits of an explicit tile, and a workspace for 16x16 tiles is enough.
+# The default tile follows the batch's 16x16 tiles (512, 1536, 6144, 16384),
+# triangles per tile (16, 24) and widths off 32 bytes: both sides of each line
+# give the bits of an explicit tile, and a workspace for 16x16 tiles is enough.
 @pytest.mark.parametrize("images,w,h,tris,layers", [
     (1, 352, 360, 300, 3), (1, 352, 376, 300, 3), (1, 352, 376, 9000, 2), (6, 256, 256, 5000, 3),
     (6, 256, 272, 5000, 3), (10, 256, 256, 200, 1), (11, 256, 256, 200, 4), (11, 256, 256, 4500, 3),
     (24, 256, 256, 5000, 3), (64, 256, 256, 300, 3), (64, 250, 256, 300, 4), (64, 256, 256, 300, 5),
-    (64, 256, 256, 6200, 3), (130, 64, 48, 40, 3)])
+    (64, 256, 256, 6200, 3), (64, 255, 256, 6200, 3), (64, 253, 256, 300, 6), (130, 64, 48, 40, 3)])
 def test_default_tile_rule(images, w, h, tris, layers, device):
   clips = []
   for i in range(min(images, 3)):
