@@ -900,7 +900,7 @@ def _pack(parts, widths, rows, device):
   ptrs = (ctypes.c_void_p * n)(*(_p(p) for p in parts))
   ws = (ctypes.c_int32 * n)(*widths)
   st = (ctypes.c_int64 * n)(*(0 if p is None else p.stride(0) for p in parts))
-  with _op("pack_columns", 1):
+  with _on_device(device), _op("pack_columns", 1):
     rc = _lib.load().dr_pack_columns(ptrs, ws, st, n, rows, _p(out), _stream(device))
   _lib.check(rc, "dr_pack_columns")
   return out
@@ -929,6 +929,9 @@ class _SplitColumns(torch.autograd.Function):
         g is not None for g in grads) else None
     if device is None:
       return None, None
+    if torch.is_grad_enabled():  # a gradient that is itself differentiated
+      return torch.cat([torch.zeros(n, w, device=device) if g is None else g
+                        for g, w in zip(grads, ctx.widths)], 1), None
     first = list(itertools.accumulate(ctx.widths[:-1], initial=0))
     if all(g is not None and g.stride() == (K, 1) for g in grads):
       whole = _one_buffer(grads, (n, K), (K, 1), first)

@@ -52,7 +52,8 @@ class _Slices(torch.autograd.Function):
     like = next((g for g in grads if g is not None), None)
     if like is None:
       return None, None
-    if all(g is not None and g.is_contiguous() for g in grads):
+    # (a gradient that is itself differentiated keeps its graph: stacked)
+    if not torch.is_grad_enabled() and all(g is not None and g.is_contiguous() for g in grads):
       n = like.numel()
       whole = kernels._one_buffer(grads, ctx.shape, (n, *like.stride()),
                                   [i * n for i in range(len(grads))])

@@ -83,3 +83,37 @@ def test_point_light_packed_gradients(rows, order, alpha, device):
     results.append((out.detach(), *torch.autograd.grad(out, [p], seed)))
   for a, b in zip(*results):
     assert torch.equal(a, b)
+
+
+# A gradient that is differentiated again (create_graph) goes through the
+# split and through the layer slices as through torch's own operations.
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 130])
+def test_second_derivatives(rows, device):
+  from diffren_gb300 import render
+  g = torch.Generator(device=device).manual_seed(rows)
+  t = torch.randn(2, rows, 1, 7, generator=g, device=device)
+
+  def columns(split):
+    def f(x):
+      a, b = split(x, [3, 4])
+      return (a ** 3).sum() + (a * a).sum() * (b ** 2).sum()
+    return f
+
+  def layers(shade):
+    def f(x):
+      y = shade(x)
+      return (y[0] * y[1]).pow(2).sum()
+    return f
+  pairs = [(columns(kernels.split_channels), columns(lambda x, w: torch.split(x, w, -1))),
+           (layers(lambda x: render._shade_layers(lambda a: a["c"] ** 2, {"c": x}, 2, False)),
+            layers(lambda x: x ** 2)),
+           (layers(lambda x: render._shade_layers(lambda a: a["c"], {"c": x}, 2, False)),
+            layers(lambda x: x))]
+  for pair in pairs:
+    second = []
+    for f in pair:
+      x = t.clone().requires_grad_()
+      first, = torch.autograd.grad(f(x), x, create_graph=True)
+      second.append(torch.autograd.grad(first.pow(2).sum(), x)[0])
+    assert (second[0] - second[1]).abs().max() <= 1e-5 * second[1].abs().max()
