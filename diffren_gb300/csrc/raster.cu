@@ -38,7 +38,8 @@ constexpr int kDefaultLargeTiles = 16;
 // times that: setup keeps theirs (RasterArgs::edges). With 144-byte records
 // of everything the fine kernel took 313 us on a 200k-triangle soup
 // (8 x 512^2), 629 on the 4 x 2048^2 terrain and 1025 on the 64-mesh ragged
-// batch, now 244, 548 and 974; setup 109, 227 and 137 us, now 94, 141 and 116.
+// batch, now 244, 548 and 974 (16x16 tiles); setup 109, 227 and 137 us, now
+// 94, 138 and 114.
 struct __align__(16) TriSetup {
   float4 v[3];
   int32_t vid[3];
@@ -423,18 +424,18 @@ __global__ void __launch_bounds__(256) tile_order_kernel(RasterArgs a, Batch B) 
   }
 }
 
-// Per chunk of up to kThreads triangles overlapping the tile, compacted to
+// Per chunk of up to kChunk triangles overlapping the tile, compacted to
 // those with at least one candidate pixel (slot = rank among them).
 struct FineSmem {
-  long long* m;          // [9][kThreads]
-  float* row;            // [9][kThreads] row-span coefficients (see row_coefficients)
-  float* vz;             // [3][kThreads]
-  float* vw;             // [3][kThreads]
-  int* tid;              // [kThreads] local triangle id
-  int* geom;             // [kThreads] x0 | y0 << 8 | width << 16 (tile-local)
-  int* off;              // [kThreads + 1] exclusive row offsets
-  long long* pxf;        // [TW] fixed-point pixel-center x
-  long long* pyf;        // [TH]
+  long long* m;          // [9][kChunk]
+  float* row;            // [9][kChunk] row-span coefficients (see row_coefficients)
+  float* vz;             // [3][kChunk]
+  float* vw;             // [3][kChunk]
+  int* tid;              // [kChunk] local triangle id
+  int* geom;             // [kChunk] x0 | y0 << 8 | width << 16 (tile-local)
+  int* off;              // [kChunk + 1] exclusive row offsets
+  int* pxf;        // [TW] fixed-point pixel-center x
+  int* pyf;        // [TH]
   unsigned long long* keys;  // [L][TW*TH]
   unsigned short* queue;  // [kThreads / 32][kQueue] candidate pixels of each warp
   unsigned char* first;  // [kThreads / 32 * TH] slot holding row 32 g, per g
@@ -444,16 +445,26 @@ struct FineSmem {
 // from one push to the next.
 constexpr int kPush = 8, kQueue = 32 * kPush + 32;
 
+// Triangles a chunk holds. Tiles above 256 pixels are taken for batches with
+// few triangles in each (default_tile), and the shared memory of 128 leaves
+// room for six blocks of 32x16 tiles and three layers per SM, where the
+// registers allow eight: the fine kernel takes 800 us on the 64-mesh ragged
+// batch with 64, 814 with 96, 883 with 128. In 16x16 tiles eight blocks fit in
+// any case and every further chunk costs: 545 us on the 4 x 2048^2 terrain
+// with 128, 574 with 96, 625 with 64.
+__host__ __device__ inline int chunk_of(int TW, int TH) { return TW * TH > 256 ? 64 : 128; }
+
 // The chunk's edge coefficients; the epilogue reuses the space for its list
 // of occupied (layer, pixel) slots (16 bits each).
 __host__ __device__ inline size_t chunk_m_bytes(int L, int TW, int TH) {
-  const size_t m = size_t(9) * kThreads * 8, list = size_t(L) * TW * TH * 2;
+  const size_t m = size_t(9) * chunk_of(TW, TH) * 8, list = size_t(L) * TW * TH * 2;
   return ((m > list ? m : list) + 7) & ~size_t(7);
 }
 
 __host__ __device__ inline size_t fine_smem_bytes(int L, int TW, int TH) {
-  return chunk_m_bytes(L, TW, TH) + size_t(TW + TH) * 8 + size_t(L) * TW * TH * 8 +
-         size_t(17) * kThreads * 4 + size_t(kThreads + 4) * 4 +
+  const size_t chunk = chunk_of(TW, TH);
+  return chunk_m_bytes(L, TW, TH) + size_t(TW + TH) * 4 + size_t(L) * TW * TH * 8 +
+         17 * chunk * 4 + (chunk + 4) * 4 +
          size_t(kThreads / 32) * kQueue * 2 + size_t(kThreads / 32) * TH;
 }
 
@@ -466,6 +477,7 @@ __host__ __device__ inline size_t fine_smem_bytes(int L, int TW, int TH) {
 // keeps every pixel that the exact test accepts. m0 = 0 gets g = +inf, so
 // that t < 0 empties the row. Coefficients from 2^43 on, whose edge functions
 // may wrap, constrain nothing.
+template <int kChunk>
 __device__ __forceinline__ void row_coefficients(const long long* m, float* row, int slot) {
   bool wraps = false;
 #pragma unroll
@@ -475,10 +487,10 @@ __device__ __forceinline__ void row_coefficients(const long long* m, float* row,
     const float a = __ll2float_rn(m[3 * i]), b = __ll2float_rn(m[3 * i + 1]),
                 c = __ll2float_rn(m[3 * i + 2]);
     const float s = fabsf(a) + fabsf(b) + fabsf(c);
-    row[(3 * i) * kThreads + slot] =
+    row[(3 * i) * kChunk + slot] =
         wraps || a == 0.0f ? __int_as_float(0x7f800000) : __fdividef(-1.0f, a);
-    row[(3 * i + 1) * kThreads + slot] = wraps ? 0.0f : b;
-    row[(3 * i + 2) * kThreads + slot] = wraps ? 1.0f : fmaf(s, 0.0625f, c * 65536.0f);
+    row[(3 * i + 1) * kChunk + slot] = wraps ? 0.0f : b;
+    row[(3 * i + 2) * kChunk + slot] = wraps ? 1.0f : fmaf(s, 0.0625f, c * 65536.0f);
   }
 }
 
@@ -671,9 +683,8 @@ __device__ __forceinline__ void fill_background(const RasterArgs& a, const TileB
 // 200k-triangle soup (8 x 512^2) and from 87 to 42 us on one 1283x717 image.
 // kFused adds the sample outputs to the epilogue. LT > 0 fixes the layer
 // count at compile time (the common L = 3), LT = 0 reads it.
-template <bool kFused, int LT>
-__global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
-                                                                             Batch B) {
+template <bool kFused, int LT, int kChunk>
+__global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a, Batch B) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_warp[kThreads / 32];
   __shared__ QueueItem s_item;
@@ -684,14 +695,14 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
     unsigned char* p = smem_raw;
     s.keys = reinterpret_cast<unsigned long long*>(p); p += size_t(L) * TP * 8;
     s.m = reinterpret_cast<long long*>(p); p += chunk_m_bytes(L, TW, TH);
-    s.pxf = reinterpret_cast<long long*>(p); p += size_t(TW) * 8;
-    s.pyf = reinterpret_cast<long long*>(p); p += size_t(TH) * 8;
-    s.row = reinterpret_cast<float*>(p); p += size_t(9) * kThreads * 4;
-    s.vz = reinterpret_cast<float*>(p); p += size_t(3) * kThreads * 4;
-    s.vw = reinterpret_cast<float*>(p); p += size_t(3) * kThreads * 4;
-    s.tid = reinterpret_cast<int*>(p); p += kThreads * 4;
-    s.geom = reinterpret_cast<int*>(p); p += kThreads * 4;
-    s.off = reinterpret_cast<int*>(p); p += (kThreads + 4) * 4;
+    s.pxf = reinterpret_cast<int*>(p); p += size_t(TW) * 4;
+    s.pyf = reinterpret_cast<int*>(p); p += size_t(TH) * 4;
+    s.row = reinterpret_cast<float*>(p); p += size_t(9) * kChunk * 4;
+    s.vz = reinterpret_cast<float*>(p); p += size_t(3) * kChunk * 4;
+    s.vw = reinterpret_cast<float*>(p); p += size_t(3) * kChunk * 4;
+    s.tid = reinterpret_cast<int*>(p); p += kChunk * 4;
+    s.geom = reinterpret_cast<int*>(p); p += kChunk * 4;
+    s.off = reinterpret_cast<int*>(p); p += (kChunk + 4) * 4;
     s.queue = reinterpret_cast<unsigned short*>(p); p += size_t(kThreads / 32) * kQueue * 2;
     s.first = p;
   }
@@ -719,8 +730,8 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
     fill_background<kFused>(a, tb, L);
     for (int p = threadIdx.x; p < L * TP; p += kThreads) s.keys[p] = kEmpty;
     for (int i = threadIdx.x; i < TW + TH; i += kThreads) {
-      if (i < TW) s.pxf[i] = pixel_center_fixed(x0 + i, W, disc);
-      else s.pyf[i - TW] = pixel_center_fixed(y0 + i - TW, H, disc);
+      if (i < TW) s.pxf[i] = int(pixel_center_fixed(x0 + i, W, disc));
+      else s.pyf[i - TW] = int(pixel_center_fixed(y0 + i - TW, H, disc));
     }
     const int bin0 = tb.bin0, nbin = tb.nbin;
     const int nlarge = a.large_count[img];
@@ -733,10 +744,10 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
     const float x_off = __int2float_rn(W) * 0.5f - 0.5f - __int2float_rn(x0);
     __syncthreads();
 
-    for (int c0 = 0; c0 < nsrc; c0 += kThreads) {
+    for (int c0 = 0; c0 < nsrc; c0 += kChunk) {
       const int i = c0 + threadIdx.x;
       int cnt = 0, g = 0, cx0 = 0, cy0 = 0, cw = 1;
-      if (i < nsrc) {
+      if ((kChunk == kThreads || threadIdx.x < kChunk) && i < nsrc) {
         g = i < nbin ? a.bins[bin0 + i] : a.large_list[tri0 + (i - nbin)];
         const int4 box = unpack_box(a.box[g]);
         cx0 = max(box.x, x0) - x0;
@@ -748,7 +759,7 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
         }
       }
       // One scan gives each triangle with candidates its compacted slot
-      // (bits 20+) and its first row (bits 0-19): at most kThreads * 128 rows
+      // (bits 20+) and its first row (bits 0-19): at most kChunk * 128 rows
       // per chunk.
       int excl;
       const int tot = block_exclusive_scan<kThreads>(cnt | (cnt > 0 ? 1 << 20 : 0), s_warp, excl);
@@ -760,14 +771,14 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
         long long mm[9];
         load_edges(a, g, v, __ldg(&st->small), mm);
 #pragma unroll
-        for (int k = 0; k < 9; ++k) s.m[k * kThreads + slot] = mm[k];
+        for (int k = 0; k < 9; ++k) s.m[k * kChunk + slot] = mm[k];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          s.vz[k * kThreads + slot] = v[k].z;
-          s.vw[k * kThreads + slot] = v[k].w;
+          s.vz[k * kChunk + slot] = v[k].z;
+          s.vw[k * kChunk + slot] = v[k].w;
         }
         s.tid[slot] = int(g - tri0);
-        row_coefficients(mm, s.row, slot);
+        row_coefficients<kChunk>(mm, s.row, slot);
         s.geom[slot] = cx0 | (cy0 << 8) | (cw << 16);
         s.off[slot] = off;
         // This triangle holds row 32 q for every q with 32 q in
@@ -805,9 +816,9 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
             float lo = -1.0e6f, hi = 1.0e6f;
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-              const float g = s.row[(3 * i) * kThreads + j];
-              const float x = fmaf(s.row[(3 * i + 1) * kThreads + j], y,
-                                   s.row[(3 * i + 2) * kThreads + j]) * g;
+              const float g = s.row[(3 * i) * kChunk + j];
+              const float x = fmaf(s.row[(3 * i + 1) * kChunk + j], y,
+                                   s.row[(3 * i + 2) * kChunk + j]) * g;
               if (g < 0.0f) lo = fmaxf(lo, x); else hi = fminf(hi, x);
             }
             const int cx0 = geom & 255;
@@ -847,14 +858,14 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a,
             const int j = int(px & 255u), ly = int((px >> 8) & 255u), lx = int(px >> 16);
             long long m[9];
 #pragma unroll
-            for (int t = 0; t < 9; ++t) m[t] = s.m[t * kThreads + j];
+            for (int t = 0; t < 9; ++t) m[t] = s.m[t * kChunk + j];
             long long e[3];
             edge_values(m, s.pxf[lx], s.pyf[ly], e);
             if (!inside(e)) continue;
             float b[3];
             barycentrics_of(e, b);
-            const float3 vz = make_float3(s.vz[j], s.vz[kThreads + j], s.vz[2 * kThreads + j]);
-            const float3 vw = make_float3(s.vw[j], s.vw[kThreads + j], s.vw[2 * kThreads + j]);
+            const float3 vz = make_float3(s.vz[j], s.vz[kChunk + j], s.vz[2 * kChunk + j]);
+            const float3 vw = make_float3(s.vw[j], s.vw[kChunk + j], s.vw[2 * kChunk + j]);
             const float z = fragment_z(b, vz, vw, disc);
             unsigned long long key;
             if (disc) {
@@ -976,10 +987,10 @@ __global__ void depth_codec_selftest_kernel(unsigned long long* out) {
 
 // Raises the fine rasterizer's dynamic shared-memory limit and computes its
 // persistent grid (resident blocks per SM x SMs) on the current device.
-template <bool kFused, int LT>
+template <bool kFused, int LT, int kChunk>
 bool prepare_fine(size_t smem, int& sms, int& per_sm, std::string& err) {
   static LaunchCache cache;
-  return prepare_launch(cache, fine_raster_kernel<kFused, LT>, kThreads, smem, sms, per_sm,
+  return prepare_launch(cache, fine_raster_kernel<kFused, LT, kChunk>, kThreads, smem, sms, per_sm,
                         "tile and layer count need more shared memory than the device has",
                         err);
 }
@@ -1020,16 +1031,18 @@ bool check_config(const dr_raster_config* cfg, int& L, int& TW, int& TH, int& la
 // tiles, 90 with 16x16; at 768x768 61 with 16x8, 83 with 16x16; from 8192 tiles
 // on 16x16 is the best (122 us, 129 with 16x8), and with fewer than 16
 // triangles a tile already above 512 (5000 triangles at 768x768: 45, 53 us).
+// The counts do not tell triangles hundreds of pixels wide, which lose by
+// it: 80k of them, 180 pixels wide at 1024x1024, take 10.3 ms, 6.7 with 16x16.
 // The threshold of the large list stays at the same number of pixels.
 // Many tiles with few triangles each are bound by the cost per tile: the
-// 64-mesh ragged batch (111k tiles) takes 1069 us with 32x16, 1174 with 16x16;
-// with more than 24 triangles a tile they are equal (terrain 770, 762). An
+// 64-mesh ragged batch (111k tiles) takes 1002 us with 32x16, 1165 with 16x16;
+// with more than 24 triangles a tile 32x16 is no better (terrain 789, 761). An
 // image whose tiles hold more than their share of all the triangles (of 912
 // resident blocks) then sets the time: one with 1531 a tile among 979k took
-// 595 us with 32x16, 518 with 16x16. Above four layers the keys of a 32x16
-// tile cost more blocks per SM than it gains (eight: 1788, 1752). Rows that do
+// 805 us with 32x16, 514 with 16x16. Above four layers the keys of a 32x16
+// tile cost more blocks per SM than it gains (eight: 498, 478). Rows that do
 // not start on 32 bytes leave partial sectors at both ends, half as many with
-// tiles twice as wide (terrain at 2047 pixels: 841 with 32x8, 878).
+// tiles twice as wide (terrain at 2047 pixels: 840 with 32x8, 876).
 void default_tile(const Batch& b, int L, int& TW, int& TH) {
   const int64_t tiles = b.tile_start[b.n], tris = b.tri_start[b.n];
   TW = TH = kDefaultTile;
@@ -1150,14 +1163,17 @@ int raster_launch(const float* vertices, const int32_t* triangles,
     }
   }
   const bool fused = so.positions != nullptr;
-  // Instantiations: fused or not, three layers or any.
+  // Instantiations: fused or not, three layers or any, chunks of 128 or 64.
   using Fine = void (*)(RasterArgs, Batch);
   using Prep = bool (*)(size_t, int&, int&, std::string&);
-  const int variant = (fused ? 2 : 0) + (L == 3 ? 1 : 0);
-  const Fine fine[4] = {fine_raster_kernel<false, 0>, fine_raster_kernel<false, 3>,
-                        fine_raster_kernel<true, 0>, fine_raster_kernel<true, 3>};
-  const Prep prep[4] = {prepare_fine<false, 0>, prepare_fine<false, 3>,
-                        prepare_fine<true, 0>, prepare_fine<true, 3>};
+  const Fine fine[8] = {fine_raster_kernel<false, 0, 128>, fine_raster_kernel<false, 3, 128>,
+                        fine_raster_kernel<true, 0, 128>,  fine_raster_kernel<true, 3, 128>,
+                        fine_raster_kernel<false, 0, 64>,  fine_raster_kernel<false, 3, 64>,
+                        fine_raster_kernel<true, 0, 64>,   fine_raster_kernel<true, 3, 64>};
+  const Prep prep[8] = {prepare_fine<false, 0, 128>, prepare_fine<false, 3, 128>,
+                        prepare_fine<true, 0, 128>,  prepare_fine<true, 3, 128>,
+                        prepare_fine<false, 0, 64>,  prepare_fine<false, 3, 64>,
+                        prepare_fine<true, 0, 64>,   prepare_fine<true, 3, 64>};
   const int TW0 = TW, TH0 = TH, large0 = large;
   for (int g0 = 0; g0 < n; g0 += DR_MAX_BATCH_INLINE) {
     const int cnt = std::min(n - g0, DR_MAX_BATCH_INLINE);
@@ -1175,6 +1191,8 @@ int raster_launch(const float* vertices, const int32_t* triangles,
       err = "workspace too small: need " + std::to_string(min_bytes) + " bytes";
       return DR_ERR_WORKSPACE_TOO_SMALL;
     }
+    const int variant =
+        (fused ? 2 : 0) + (L == 3 ? 1 : 0) + (chunk_of(TW, TH) == 64 ? 4 : 0);
     const size_t smem = fine_smem_bytes(L, TW, TH);
     int sms = 0, per_sm = 0;
     if (!prep[variant](smem, sms, per_sm, err)) return DR_ERR_INVALID_ARGUMENT;

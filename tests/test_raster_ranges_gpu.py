@@ -96,3 +96,24 @@ def test_default_tile_rule(images, w, h, tris, layers, device):
     if ok:
       for a, b in zip(out, want):
         assert torch.equal(a, b)
+
+
+# Tiles above 256 pixels take triangles 64 at a time, the others 128: the same
+# bits with one triangle less and more than whole chunks in a tile.
+@pytest.mark.parametrize("count", [1, 63, 64, 65, 127, 128, 129, 257])
+@pytest.mark.parametrize("layers", [1, 3, 16])
+def test_chunk_of_large_tiles(count, layers, device):
+  g = torch.Generator(device=device).manual_seed(count)
+  w, h = 37, 29
+  clip = torch.rand(3 * count, 4, generator=g, device=device) * 2 - 1
+  clip[:, 3] = 1.0
+  tri = torch.arange(3 * count, dtype=torch.int32, device=device).view(-1, 3)
+  batch = kernels.ImageBatch([w], [h], [3 * count], [count])
+  out = [kernels.rasterize_packed(clip, tri, batch, kernels.raster_config(
+      layers, culling, _lib.DR_DEPTH_DISCRETIZED, tile, large))
+         for culling in (0, 1) for large in (1, 16)
+         for tile in ((16, 16), (32, 16), (32, 32), (17, 16), (64, 5))]
+  for k in range(0, len(out), 5):
+    for got in out[k + 1:k + 5]:
+      for a, b in zip(got, out[k]):
+        assert torch.equal(a, b)
