@@ -445,24 +445,27 @@ struct FineSmem {
 // from one push to the next.
 constexpr int kPush = 8, kQueue = 32 * kPush + 32;
 
-// Triangles a chunk holds. Tiles above 256 pixels are taken for batches with
-// few triangles in each (default_tile), and the shared memory of 128 leaves
-// room for six blocks of 32x16 tiles and three layers per SM, where the
-// registers allow eight: the fine kernel takes 800 us on the 64-mesh ragged
-// batch with 64, 814 with 96, 883 with 128. In 16x16 tiles eight blocks fit in
-// any case and every further chunk costs: 545 us on the 4 x 2048^2 terrain
-// with 128, 574 with 96, 625 with 64.
-__host__ __device__ inline int chunk_of(int TW, int TH) { return TW * TH > 256 ? 64 : 128; }
+// Triangles a chunk holds. Up to 768 keys (16x16 pixels of three layers) eight
+// blocks of 128 fit an SM's shared memory, as the registers allow, and every
+// further chunk costs: the fine kernel takes 545 us on the 4 x 2048^2 terrain
+// with 128, 574 with 96, 625 with 64. Above, 64 keep eight blocks up to eight
+// layers of 16x16, where 128 leave seven to five: 800 us on the 64-mesh
+// ragged batch in 32x16 tiles (883 with 128); setup to fine kernel for a
+// 100k-triangle sphere (8 x 1024^2) 454 us (466) at four layers, 535 (579) at
+// six, 612 (649) at eight.
+__host__ __device__ inline int chunk_of(int L, int TW, int TH) {
+  return L * TW * TH > 768 ? 64 : 128;
+}
 
 // The chunk's edge coefficients; the epilogue reuses the space for its list
 // of occupied (layer, pixel) slots (16 bits each).
 __host__ __device__ inline size_t chunk_m_bytes(int L, int TW, int TH) {
-  const size_t m = size_t(9) * chunk_of(TW, TH) * 8, list = size_t(L) * TW * TH * 2;
+  const size_t m = size_t(9) * chunk_of(L, TW, TH) * 8, list = size_t(L) * TW * TH * 2;
   return ((m > list ? m : list) + 7) & ~size_t(7);
 }
 
 __host__ __device__ inline size_t fine_smem_bytes(int L, int TW, int TH) {
-  const size_t chunk = chunk_of(TW, TH);
+  const size_t chunk = chunk_of(L, TW, TH);
   return chunk_m_bytes(L, TW, TH) + size_t(TW + TH) * 4 + size_t(L) * TW * TH * 8 +
          17 * chunk * 4 + (chunk + 4) * 4 +
          size_t(kThreads / 32) * kQueue * 2 + size_t(kThreads / 32) * TH;
@@ -1040,7 +1043,7 @@ bool check_config(const dr_raster_config* cfg, int& L, int& TW, int& TH, int& la
 // image whose tiles hold more than their share of all the triangles (of 912
 // resident blocks) then sets the time: one with 1531 a tile among 979k took
 // 805 us with 32x16, 514 with 16x16. Above four layers the keys of a 32x16
-// tile cost more blocks per SM than it gains (eight: 498, 478). Rows that do
+// tile cost more blocks per SM than it gains (eight: 744, 612 on a sphere). Rows that do
 // not start on 32 bytes leave partial sectors at both ends, half as many with
 // tiles twice as wide (terrain at 2047 pixels: 840 with 32x8, 876).
 void default_tile(const Batch& b, int L, int& TW, int& TH) {
@@ -1192,7 +1195,7 @@ int raster_launch(const float* vertices, const int32_t* triangles,
       return DR_ERR_WORKSPACE_TOO_SMALL;
     }
     const int variant =
-        (fused ? 2 : 0) + (L == 3 ? 1 : 0) + (chunk_of(TW, TH) == 64 ? 4 : 0);
+        (fused ? 2 : 0) + (L == 3 ? 1 : 0) + (chunk_of(L, TW, TH) == 64 ? 4 : 0);
     const size_t smem = fine_smem_bytes(L, TW, TH);
     int sms = 0, per_sm = 0;
     if (!prep[variant](smem, sms, per_sm, err)) return DR_ERR_INVALID_ARGUMENT;

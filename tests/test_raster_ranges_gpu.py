@@ -98,10 +98,10 @@ def test_default_tile_rule(images, w, h, tris, layers, device):
         assert torch.equal(a, b)
 
 
-# Tiles above 256 pixels take triangles 64 at a time, the others 128: the same
-# bits with one triangle less and more than whole chunks in a tile.
+# Tiles with more than 768 keys take triangles 64 at a time, the others 128: the
+# same bits with one triangle less and more than whole chunks in a tile.
 @pytest.mark.parametrize("count", [1, 63, 64, 65, 127, 128, 129, 257])
-@pytest.mark.parametrize("layers", [1, 3, 16])
+@pytest.mark.parametrize("layers", [1, 3, 4, 16])
 def test_chunk_of_large_tiles(count, layers, device):
   g = torch.Generator(device=device).manual_seed(count)
   w, h = 37, 29
