@@ -269,7 +269,7 @@ class ClockSampler:
 # profiles/): setup + tile scan + binning + fine raster;
 # splat forward; splat backward; samples VJP. Traffic grows with the layer
 # samples, so the full workload's traffic is this times its samples.
-TRAFFIC_PER_SAMPLE = {"raster": 32.98, "splat_fwd": 22.61, "splat_bwd": 31.73,
+TRAFFIC_PER_SAMPLE = {"raster": 32.49, "splat_fwd": 22.62, "splat_bwd": 29.99,
                       "samples_bwd": 22.92}
 
 

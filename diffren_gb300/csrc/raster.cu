@@ -434,8 +434,8 @@ struct FineSmem {
   int* tid;              // [kChunk] local triangle id
   int* geom;             // [kChunk] x0 | y0 << 8 | width << 16 (tile-local)
   int* off;              // [kChunk + 1] exclusive row offsets
-  int* pxf;        // [TW] fixed-point pixel-center x
-  int* pyf;        // [TH]
+  int* pxf;              // [TW] fixed-point pixel-center x
+  int* pyf;              // [TH]
   unsigned long long* keys;  // [L][TW*TH]
   unsigned short* queue;  // [kThreads / 32][kQueue] candidate pixels of each warp
   unsigned char* first;  // [kThreads / 32 * TH] slot holding row 32 g, per g
@@ -1040,8 +1040,8 @@ bool check_config(const dr_raster_config* cfg, int& L, int& TW, int& TH, int& la
 // Many tiles with few triangles each are bound by the cost per tile: the
 // 64-mesh ragged batch (111k tiles) takes 1002 us with 32x16, 1165 with 16x16;
 // with more than 24 triangles a tile 32x16 is no better (terrain 789, 761). An
-// image whose tiles hold more than their share of all the triangles (of 912
-// resident blocks) then sets the time: one with 1531 a tile among 979k took
+// image whose tiles hold more than 1/912 of all the triangles each (about a
+// block's share) then sets the time: one with 1531 a tile among 979k took
 // 805 us with 32x16, 514 with 16x16. Above four layers the keys of a 32x16
 // tile cost more blocks per SM than it gains (eight: 744, 612 on a sphere). Rows that do
 // not start on 32 bytes leave partial sectors at both ends, half as many with
