@@ -146,9 +146,9 @@ __global__ void __launch_bounds__(256) texture_fwd_kernel(TexArgs a) {
 }
 
 // The common cases on 32-bit texel indices: up to four channels, edge padding,
-// a texture of fewer than 2^29 texels, 8-byte aligned uv, and for four
-// channels 16-byte aligned texture and output. Same operations and order as
-// texture_fwd_kernel. Each thread takes two points a block's width apart, so
+// a texture of fewer than 2^29 texels and sides up to 2^24 (fits_foot32), 8-byte
+// aligned uv, and for four channels 16-byte aligned texture and output. Same
+// operations and order as texture_fwd_kernel. Each thread takes two points a block's width apart, so
 // that their coordinate loads, and then their texel loads, are in flight
 // together, and six blocks share an SM: the kernels wait on those loads (the
 // 50 M points of the 4 x 2048^2 terrain, forward and backward, take 76 us less
@@ -156,6 +156,14 @@ __global__ void __launch_bounds__(256) texture_fwd_kernel(TexArgs a) {
 // more). Three channels: 16 and 48 us for 1.5 M points, 19 and 69 us in the
 // general kernels, whose backward issues three reductions a texel, not two.
 constexpr int kPoints = 2;
+
+// Padding and texture sizes that foot32's indexes stay inside. axis_of clips the
+// floor index to the size as a float, exact up to 2^24; a longer side's may round
+// past it (16777219 to 16777220), a row that foot32's one-sided clamps would read.
+bool fits_foot32(int H, int W, int C, int flags) {
+  return C <= 4 && !(flags & DR_TEXTURE_PAD_ZERO) && H <= (1 << 24) && W <= (1 << 24) &&
+         int64_t(H) * W < (int64_t(1) << 29);
+}
 
 struct Foot32 {
   Axis r, c;
@@ -442,8 +450,8 @@ int texture_fwd_launch(const float* uv, int64_t n, const float* tex, int H, int 
   if (!out) { err = "out must be non-null"; return DR_ERR_INVALID_ARGUMENT; }
   TexArgs a{uv, tex, H, W, C, flags, n, out, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
   const uintptr_t wide = reinterpret_cast<uintptr_t>(tex) | reinterpret_cast<uintptr_t>(out);
-  if (C <= 4 && !(flags & DR_TEXTURE_PAD_ZERO) && int64_t(H) * W < (int64_t(1) << 29) &&
-      (reinterpret_cast<uintptr_t>(uv) & 7) == 0 && (C != 4 || (wide & 15) == 0)) {
+  if (fits_foot32(H, W, C, flags) && (reinterpret_cast<uintptr_t>(uv) & 7) == 0 &&
+      (C != 4 || (wide & 15) == 0)) {
     using Kernel = void (*)(TexArgs);
     const Kernel kernels[4] = {texture_fwd32_kernel<1>, texture_fwd32_kernel<2>,
                                texture_fwd32_kernel<3>, texture_fwd32_kernel<4>};
@@ -499,8 +507,7 @@ int texture_bwd_launch(const float* d_out, const float* uv, int64_t n, const flo
                           reinterpret_cast<uintptr_t>(d_tex);
   const uintptr_t wide = reinterpret_cast<uintptr_t>(tex) | reinterpret_cast<uintptr_t>(d_out) |
                          reinterpret_cast<uintptr_t>(d_tex);
-  if (C <= 4 && !(flags & DR_TEXTURE_PAD_ZERO) && int64_t(H) * W < (int64_t(1) << 29) &&
-      (pairs & 7) == 0 && (C != 4 || (wide & 15) == 0)) {
+  if (fits_foot32(H, W, C, flags) && (pairs & 7) == 0 && (C != 4 || (wide & 15) == 0)) {
     using Kernel = void (*)(TexArgs);
     const Kernel kernels[4] = {texture_bwd32_kernel<1>, texture_bwd32_kernel<2>,
                                texture_bwd32_kernel<3>, texture_bwd32_kernel<4>};

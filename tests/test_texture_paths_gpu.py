@@ -42,3 +42,26 @@ def test_texture_dispatch(channels, points, offset, device):
   # largest magnitude.
   for x, y in zip(got, want):
     assert (x.cpu().double() - y).abs().max() <= 1e-4 * y.abs().max()
+
+
+# float32 rounds sides above 2^24 to even numbers: 2^24 + 3 becomes 2^24 + 4, one
+# past the last padded texel. Coordinates at and beyond the far edge are the last
+# texel and its gradient, those at the near edge the first.
+@pytest.mark.parametrize("side", [2**24 - 1, 2**24, 2**24 + 3])
+@pytest.mark.parametrize("channels,rows", [(1, True), (1, False), (2, True), (3, False), (4, True)])
+def test_far_edge_of_long_sides(side, channels, rows, device):
+  far = [1.0, 1.25, 2.0, 1e9, float("inf")]
+  at = torch.tensor([0.0, -1.0] + far, device=device)
+  mid = torch.full_like(at, 0.5)
+  uv = torch.stack((mid, at) if rows else (at, mid), -1).requires_grad_()
+  tex = torch.zeros(side, channels, device=device)
+  tex[0] = torch.arange(1, channels + 1, device=device)
+  tex[-1] = -torch.arange(3, channels + 3, device=device)
+  tex = (tex[:, None] if rows else tex[None]).requires_grad_()
+  ends = tex.detach().view(side, channels)[[0, 0] + [-1] * len(far)]
+  out = shaders.texture_map(uv, tex)
+  assert torch.equal(out, ends)
+  g = torch.arange(1, out.numel() + 1, device=device).float().view_as(out)
+  d_tex = torch.autograd.grad(out, tex, g)[0].view(side, channels)
+  assert torch.equal(d_tex[0], g[:2].sum(0)) and torch.equal(d_tex[-1], g[2:].sum(0))
+  assert int((d_tex != 0).sum()) == 2 * channels
