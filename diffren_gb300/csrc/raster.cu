@@ -1070,6 +1070,15 @@ void default_tile(const Batch& b, int L, int& TW, int& TH) {
   }
 }
 
+// Tiles a triangle may take bins in. Bin positions are 32-bit integers, so all
+// triangles together get fewer than 2^31: from 134 million on at the default 16,
+// the threshold falls (to 1 at the 2^31 triangles that make_batch refuses).
+// Triangles above it go to the large list, whatever their size, and the results
+// do not depend on it.
+int bounded_large(int large, int64_t tris) {
+  return tris > 0 ? int(std::min(int64_t(large), INT32_MAX / tris)) : large;
+}
+
 // The batch table of one group with its tiles, and the workspace it needs.
 // With a tile by the rule that workspace may exceed the 16x16 one, which is
 // then enough too (at 16x16): `min_bytes` is what a call must bring.
@@ -1077,6 +1086,7 @@ bool group_batch(const dr_image_desc* images, int n, const dr_raster_config* cfg
                  size_t ws_bytes, int& TW, int& TH, int& large, Batch& b, Layout& lay,
                  size_t& min_bytes, std::string& err) {
   if (!make_batch(images, n, L, TW, TH, b, err)) return false;
+  large = bounded_large(large, b.tri_start[n]);
   lay = make_layout(b.tri_start[n], b.tile_start[n], n, large);
   min_bytes = lay.total;
   if (cfg->tile_width > 0 || cfg->tile_height > 0) return true;
@@ -1089,6 +1099,7 @@ bool group_batch(const dr_image_desc* images, int n, const dr_raster_config* cfg
   int ruled_large = large;
   if (cfg->large_tiles <= 0)
     ruled_large = std::max(large, large * kDefaultTile * kDefaultTile / (w * h));
+  if (ruled_large != bounded_large(ruled_large, b.tri_start[n])) return true;
   const Layout l = make_layout(ruled.tri_start[n], ruled.tile_start[n], n, ruled_large);
   if (l.total > ws_bytes) return true;
   b = ruled;

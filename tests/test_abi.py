@@ -74,6 +74,27 @@ def test_workspace_grows_with_triangles_and_tiles():
   assert f(big) > f(small) and f(wide) > f(small)
 
 
+@pytest.mark.parametrize("tris", [1000, 33 << 20, 40_000_000, 128 << 20, 134_217_728, 1 << 30,
+                                  (1 << 31) - 1])
+@pytest.mark.parametrize("w,h", [(64, 64), (512, 256), (640, 512), (1024, 512), (4096, 4096)])
+def test_bins_fit_32_bits(tris, w, h):
+  """Bin positions are int32: whatever the tile and the large-triangle
+  threshold, the bins of all triangles together stay below 2^31. A threshold
+  of 1 differs from another one by the bins alone (4 bytes each)."""
+  lib = _lib.load()
+  b = kernels.ImageBatch.single(w, h, 3, tris)
+
+  def need(tile, large):
+    cfg = kernels.raster_config(3, 1, 0, tile, large)
+    n = lib.dr_rasterize_batch_workspace_bytes(b.ptr, 1, ctypes.byref(cfg))
+    assert n > 0
+    return n
+  for tile in ((0, 0), (8, 8), (16, 16)):
+    for large in (0, 1, 16, 64, 2000):
+      bins = tris + (need(tile, large) - need(tile, 1)) // 4
+      assert bins < (1 << 31) + 64  # 256 bytes of alignment
+
+
 def test_entry_points_reject_bad_arguments_without_gpu_work():
   lib = _lib.load()
   b = kernels.ImageBatch.single(8, 8, 3, 1)
