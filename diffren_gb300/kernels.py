@@ -104,8 +104,16 @@ def _p(t):
 
 
 def _stream(device=None):
-  """Handle of the current stream of a device (torch.device or None)."""
-  index = None if device is None else device.index
+  """Handle of the current stream of a device (None: the current one). Every
+  op asks for it before its call, so this is where host tensors are refused
+  that no check before it caught."""
+  index = None
+  if device is not None:
+    if not isinstance(device, torch.device):
+      device = torch.device(device)
+    if device.type != "cuda":
+      raise ValueError("diffren_gb300 ops take CUDA tensors; got a %s device" % device)
+    index = device.index
   if index is None:
     index = torch.cuda.current_device()
   return torch._C._cuda_getCurrentRawStream(index)

@@ -28,6 +28,39 @@ def test_image_batch_offsets_and_views():
     kernels.ImageBatch([0], [1], [1], [1])
 
 
+def test_host_tensors_are_refused():
+  """Host tensors never reach a kernel: entry points without a check of their
+  own are stopped where they ask for the device's stream."""
+  from diffren_gb300 import splat
+  for device in (torch.device("cpu"), "cpu"):
+    with pytest.raises(ValueError, match="take CUDA tensors"):
+      kernels._stream(device)
+    with pytest.raises(ValueError, match="take CUDA tensors"):
+      kernels.read_error_flags(torch.zeros(256, dtype=torch.uint8), device)
+  with pytest.raises(ValueError, match="take CUDA tensors"):
+    kernels.default_workspace(torch.device("cpu"))
+  with pytest.raises(ValueError, match="take CUDA tensors"):
+    splat.splat_at_pixel_centers(torch.zeros(2, 4, 5, 3), torch.zeros(2, 4, 5, 4),
+                                 torch.ones(2, 4, 5, 1))
+  batch = kernels.ImageBatch.single(5, 4, 3, 1)
+  tri = torch.zeros(1, 3, dtype=torch.int32)
+  ids, z, bary = torch.zeros(20, dtype=torch.int32), torch.zeros(20), torch.zeros(20, 3)
+  with pytest.raises(ValueError, match="take CUDA tensors"):
+    kernels.interpolate_packed(torch.zeros(3, 4), bary, tri, ids, z, batch, 1)
+  with pytest.raises(ValueError, match="take CUDA tensors"):
+    kernels.diff_barycentrics_packed(torch.zeros(3, 4), tri, ids, z, batch, 1)
+  with pytest.raises(ValueError, match="take CUDA tensors"):
+    kernels.splat_positions_packed(torch.zeros(3, 4), bary, tri, ids, z, batch, 1)
+
+
+@pytest.mark.gpu
+def test_streams_of_every_form_of_device(device):
+  with torch.cuda.stream(torch.cuda.Stream(device)):
+    want = torch.cuda.current_stream(device).cuda_stream
+    for d in (None, device, torch.device("cuda"), "cuda", "cuda:0", 0):
+      assert kernels._stream(d) == want
+
+
 def test_render_validates_before_gpu_work():
   v = torch.zeros(3, 3)
   t = torch.zeros(1, 3, dtype=torch.int32)
