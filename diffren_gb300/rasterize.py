@@ -77,14 +77,15 @@ class Geometry:
     T = triangles.shape[-2]
     self.batch = kernels.ImageBatch([image_width] * B, [image_height] * B, [V] * B,
                                     [T] * B)
-    if self.batched:
+    if (vertices.dim() == triangles.dim() == 2 and triangles.shape[1] == 3 and
+        (camera is None or camera.shape == (4, 4))):  # one image: packed as it is
+      v, t = vertices, triangles
+    else:
       v = vertices.expand(B, *vertices.shape[-2:]) if vertices.dim() == 2 else vertices
       t = triangles.expand(B, T, 3) if triangles.dim() == 2 else triangles
       v, t = v.reshape(B * V, vertices.shape[-1]), t.reshape(B * T, 3)
       if camera is not None and camera.dim() == 2:
         camera = camera.expand(B, 4, 4)
-    else:
-      v, t = vertices, triangles
     self.world = v.float()
     self.triangles_packed = t.to(torch.int32).contiguous()
     self.triangles = triangles

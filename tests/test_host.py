@@ -53,6 +53,27 @@ def test_host_tensors_are_refused():
     kernels.splat_positions_packed(torch.zeros(3, 4), bary, tri, ids, z, batch, 1)
 
 
+def test_geometry_takes_the_shapes_it_packs(monkeypatch):
+  """[T, 3] triangles and a [4, 4] camera, whatever checked them before; ranks
+  that hold the same elements are packed."""
+  monkeypatch.setattr(rasterize, "_device", lambda *a: torch.device("cpu"))
+  monkeypatch.setattr(kernels, "transform", lambda v, m, batch: (v, m))
+  clip = torch.arange(12.0).view(3, 4)
+  tri = torch.tensor([[0, 1, 2]])
+  for v, t in ((clip, tri), (clip[None, None], tri), (clip, tri[None, None])):
+    geom = rasterize.Geometry(v, t, None, 8, 8)
+    assert torch.equal(geom.clip, clip) and not geom.batched
+    assert torch.equal(geom.triangles_packed, tri.int())
+  for shape in ((1, 4), (1, 2), (2, 6)):
+    with pytest.raises(RuntimeError):
+      rasterize.Geometry(clip, torch.zeros(shape, dtype=torch.int32), None, 8, 8)
+  for shape in ((2, 8), (8, 2), (3, 4), (16, 1)):
+    with pytest.raises(RuntimeError):
+      rasterize.Geometry(clip, tri, torch.zeros(shape), 8, 8)
+  for m in (torch.eye(4), torch.eye(4)[None]):
+    assert rasterize.Geometry(clip, tri, m, 8, 8).clip[1].numel() == 16
+
+
 @pytest.mark.gpu
 def test_streams_of_every_form_of_device(device):
   with torch.cuda.stream(torch.cuda.Stream(device)):
