@@ -138,19 +138,19 @@ def _row_stride(t):
   return 3 if rows.shape[0] <= 1 else rows.stride(0)
 
 
+def _rows_of_three(t):
+  """(t or a contiguous float32 copy, its row stride) for the kernels."""
+  st = _row_stride(t)
+  return (t.float().contiguous(), 3) if st is None or st < 3 else (t, st)
+
+
 class _PointLight(torch.autograd.Function):
   """dr_point_light_fwd / _bwd: the whole shader in one kernel each way."""
 
   @staticmethod
   def forward(ctx, diffuse, normals, positions, params, out_channels):
     lib = _lib.load()
-    ins = []
-    for t in (diffuse, normals, positions):
-      st = _row_stride(t)
-      if st is None or st < 3:
-        t, st = t.float().contiguous(), 3
-      ins.append((t, st))
-    (dif, sd), (nrm, sn), (pos, sp) = ins
+    (dif, sd), (nrm, sn), (pos, sp) = map(_rows_of_three, (diffuse, normals, positions))
     n = dif.numel() // 3 if dif.dim() > 0 else 0
     out = torch.empty(n, out_channels, dtype=torch.float32, device=dif.device)
     with kernels._op("point_light", 1):
@@ -159,19 +159,19 @@ class _PointLight(torch.autograd.Function):
                                   kernels._stream(dif.device))
     _lib.check(rc, "dr_point_light_fwd")
     ctx.save_for_backward(dif, nrm, pos)
-    ctx.strides, ctx.params, ctx.oc, ctx.n = (sd, sn, sp), params, out_channels, n
+    ctx.params, ctx.oc, ctx.n = params, out_channels, n
     ctx.shapes = (diffuse.shape, normals.shape, positions.shape)
     return out.view(*diffuse.shape[:-1], out_channels)
 
   @staticmethod
   def backward(ctx, d_out):
-    dif, nrm, pos = ctx.saved_tensors
+    # (saved-tensor hooks give tensors of their own strides back)
+    (dif, sd), (nrm, sn), (pos, sp) = map(_rows_of_three, ctx.saved_tensors)
     lib = _lib.load()
     need = ctx.needs_input_grad[:3]
     if not any(need):
       return None, None, None, None, None
     d_out = d_out.float().contiguous()
-    sd, sn, sp = ctx.strides
     # Inputs that are the columns of one packed buffer get their gradients as
     # the columns of another, which the split's gradient then takes as it is.
     start = min(t.storage_offset() for t in (dif, nrm, pos))

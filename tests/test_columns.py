@@ -85,6 +85,27 @@ def test_point_light_packed_gradients(rows, order, alpha, device):
     assert torch.equal(a, b)
 
 
+# Saved-tensor hooks hand back tensors with strides of their own: the gradients
+# of packed columns are those without hooks.
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [2, 300])
+@pytest.mark.parametrize("unpack", [lambda t: t.contiguous(), lambda t: t.t().contiguous().t(),
+                                    lambda t: torch.cat([t, t], 1)[:, 3:]])
+def test_point_light_under_saved_tensor_hooks(rows, unpack, device):
+  from diffren_gb300 import shaders
+  g = torch.Generator(device=device).manual_seed(rows)
+  packed = torch.randn(rows, 9, generator=g, device=device)
+  seed = torch.randn(rows, 3, generator=g, device=device)
+
+  def grad(hooks):
+    p = packed.clone().requires_grad_()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, hooks):
+      out = shaders.point_light(*kernels.split_channels(p, [3, 3, 3]), (2.0, 2.0, 2.0), ks=0.4,
+                                ns=3.0)
+      return torch.autograd.grad(out, p, seed)[0]
+  assert torch.equal(grad(unpack), grad(lambda t: t))
+
+
 # A gradient that is differentiated again (create_graph) goes through the
 # split and through the layer slices as through torch's own operations.
 @pytest.mark.gpu
