@@ -817,6 +817,14 @@ def splat_positions_packed(clip, bary, triangles, ids, z, batch, num_layers):
   return _Positions.apply(clip, bary, triangles, ids, z, batch, num_layers)
 
 
+def _saved_buffer(saved):
+  """The splat's saved accumulators for its VJP. Their layout follows the
+  buffer's 16-byte alignment, which torch.empty gave the forward and a
+  saved-tensor hook need not keep."""
+  saved = saved.contiguous()
+  return saved.clone() if saved.data_ptr() % 16 else saved
+
+
 class _Splat(torch.autograd.Function):
 
   @staticmethod
@@ -872,6 +880,8 @@ class _Splat(torch.autograd.Function):
     d_out = d_out.contiguous()
     if d_out.data_ptr() % 16:
       d_out = d_out.clone()
+    if saved is not None:
+      saved = _saved_buffer(saved)
     d_colors = torch.empty_like(colors)
     d_pos = torch.empty_like(positions)
     flags = _lib.DR_SPLAT_FOREGROUND_GRADIENTS if ctx.fg_grads else 0

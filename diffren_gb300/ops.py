@@ -82,10 +82,11 @@ def splat_bwd(d_out: torch.Tensor, positions: torch.Tensor, colors: torch.Tensor
   pos = positions.reshape(-1, 4).contiguous()
   col = colors.reshape(-1, C).contiguous()
   z = z_buffer.reshape(-1).contiguous()
+  saved = kernels._saved_buffer(saved)
   d_pos = torch.zeros_like(pos)  # background samples get no gradient
   d_col = torch.empty_like(col)
   rc = lib.dr_splat_bwd(kernels._p(d_out.contiguous()), kernels._p(pos), kernels._p(z),
-                        kernels._p(col), kernels._p(saved.contiguous()), C, batch.ptr, 1, L,
+                        kernels._p(col), kernels._p(saved), C, batch.ptr, 1, L,
                         kernels._p(d_col), kernels._p(d_pos), kernels._stream(colors.device))
   _lib.check(rc, "dr_splat_bwd")
   return d_pos.view(L, H, W, 4), d_col.view(L, H, W, C)

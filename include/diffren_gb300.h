@@ -504,7 +504,8 @@ int dr_vertex_normals_csr_bwd(const float* d_normals, const float* vertices,
  * foreground: one plane of P pixels per value, or, for four channels in a
  * 16-byte aligned buffer, four planes of 16 bytes per pixel (nullable; the
  * planes are written only near foreground samples, where dr_splat_bwd reads
- * them; the buffer belongs to the library between the calls); accum and
+ * them; the buffer belongs to the library between the calls, and a copy that
+ * dr_splat_bwd gets instead is 16-byte aligned if the buffer was); accum and
  * normalized [3, H, W, C] are
  * the reference's debugging buffers (nullable). With C % 4 == 0 the color
  * and output buffers must be 16-byte aligned. */

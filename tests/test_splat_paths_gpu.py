@@ -127,3 +127,45 @@ def test_saved_planes_aligned_and_not(layers, listed, device):
     results.append((out, d_c, d_p))
   for a, b in zip(*results):
     assert torch.equal(a, b) and torch.count_nonzero(a) > 0
+
+
+# The layout follows the buffer's alignment in the forward: a saved-tensor hook
+# (or a caller of the registered op) that hands the backward a copy elsewhere
+# gets the same gradients.
+@pytest.mark.parametrize("layers", [1, 2, 3, 4])
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_saved_buffer_moved_off_its_alignment(layers, offset, device):
+  from diffren_gb300 import ops
+  w, h, C = 70, 33, 4
+  g = torch.Generator(device=device).manual_seed(layers)
+  rand = lambda *s: torch.rand(*s, generator=g, device=device)
+  fg = torch.arange(layers, device=device)[:, None, None] < (rand(h, w) * (layers + 1)).long()
+  z = torch.where(fg, 0.5, 1.0).contiguous()
+  pos = torch.zeros(layers, h, w, 4, device=device)
+  pos[..., 0] = torch.arange(w, device=device) + rand(layers, h, w)
+  pos[..., 1] = torch.arange(h, device=device)[:, None] + rand(layers, h, w)
+  pos[..., 2] = torch.where(fg, rand(layers, h, w), 1.0)
+  pos[..., 3] = fg.float()
+  colors = rand(layers, h, w, C)
+  d_out = torch.randn(h, w, C, generator=g, device=device)
+  batch = kernels.ImageBatch.single(w, h, 0, 0)
+  rows = 3 * (C + 1) + 2
+
+  def moved(t):
+    if t.shape[0] != rows:
+      return t
+    buf = torch.empty(t.numel() + offset, device=device)
+    return buf[offset:].view_as(t).copy_(t)
+
+  def grads(unpack):
+    p, c = pos.view(-1, 4).clone().requires_grad_(), colors.view(-1, C).clone().requires_grad_()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+      out = kernels.splat_packed(p, c, batch, layers, z=z.view(-1))
+      d_p, d_c = torch.autograd.grad(out, [p, c], d_out.view(-1, C))
+    return torch.where(fg.view(-1, 1), d_p, 0.0), d_c
+  want = grads(lambda t: t)
+  for a, b in zip(grads(moved), want):
+    assert torch.equal(a, b) and torch.count_nonzero(a) > 0
+  image, saved = ops.splat_fwd(pos, colors, z)
+  d_p, d_c = ops.splat_bwd(d_out, pos, colors, z, moved(saved))
+  assert torch.equal(d_c.view(-1, C), want[1]) and torch.equal(d_p.view(-1, 4), want[0])
