@@ -896,10 +896,10 @@ class _Splat(torch.autograd.Function):
 
 def _one_buffer(parts, shape, stride, step):
   """The tensor of `shape` and `stride` whose pieces are `parts`, the i-th
-  starting step[i] floats after the first, when they lie so in one buffer;
-  None otherwise."""
+  starting step[i] floats after the first, when they lie so in one buffer, on
+  16 bytes as the kernels that read rows of four take it; None otherwise."""
   first = parts[0]
-  if first is None:
+  if first is None or first.data_ptr() % 16:
     return None
   base = first.untyped_storage().data_ptr()
   for p, d in zip(parts, step):

@@ -49,6 +49,35 @@ def test_pack_and_split(rows, widths, device):
         assert torch.equal(x, grads[i] if i in which else torch.zeros_like(grads[i]))
 
 
+# Gradients that share a buffer are that buffer where it starts on 16 bytes, and
+# are packed into one that does elsewhere (float offsets 1 to 3).
+@pytest.mark.parametrize("offset", [0, 1, 2, 3, 4])
+def test_one_buffer_is_aligned(offset):
+  whole = torch.arange(40.0 + offset)[offset:].view(10, 4)
+  got = kernels._one_buffer(torch.split(whole, [3, 1], 1), (10, 4), (4, 1), [0, 3])
+  assert got is None if offset % 4 else torch.equal(got, whole)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("offset", [0, 1, 2, 4])
+def test_split_gradients_off_alignment_reach_the_rasterizer(offset, device):
+  w, h, layers = 24, 20, 2
+  clip = torch.tensor([[-0.9, -0.9, 0.1, 1.0], [0.9, -0.8, 0.2, 1.0], [0.0, 0.9, 0.3, 1.0]],
+                      device=device)
+  tri = torch.tensor([[0, 1, 2]], dtype=torch.int32, device=device)
+  attr = torch.rand(3, 4, device=device).requires_grad_()
+  cfg = kernels.raster_config(layers, 0, _lib.DR_DEPTH_DISCRETIZED)
+  batch = kernels.ImageBatch.single(w, h, 3, 1)
+  out, _, _, z, bary = kernels.rasterize_interpolate_packed(attr, clip, tri, batch, cfg,
+                                                            kernels.Workspace(device))
+  n = out.shape[0]
+  d = torch.ones(4 * n + offset, device=device)[offset:].view(n, 4)
+  got = torch.autograd.grad(kernels.split_channels(out, [3, 1]), attr, torch.split(d, [3, 1], 1))[0]
+  want = bary[z != 1.0].double().sum(0)  # the same for every channel
+  # sums of some hundred products in [0, 1]
+  assert (got.double() - want[:, None]).abs().max() <= 1e-5 * want.max() and want.min() > 10
+
+
 @pytest.mark.gpu
 def test_pack_and_split_forward_mode(device):
   import torch.autograd.forward_ad as fwAD
