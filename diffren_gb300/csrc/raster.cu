@@ -1028,45 +1028,48 @@ bool check_config(const dr_raster_config* cfg, int& L, int& TW, int& TH, int& la
 }
 
 // Tile of a group of images whose configuration gives none, from its table
-// with 16x16 tiles. Few tiles leave most of the 1216 resident blocks idle,
-// and where there are triangles enough smaller tiles spread them: setup to
-// fine kernel for a 100k-triangle sphere takes 57 us at 256x256 with 8x8
-// tiles, 90 with 16x16; at 768x768 61 with 16x8, 83 with 16x16; from 8192 tiles
-// on 16x16 is the best (122 us, 129 with 16x8), and with fewer than 16
-// triangles a tile already above 512 (5000 triangles at 768x768: 45, 53 us).
-// The counts do not tell triangles hundreds of pixels wide, which lose by
-// it: 80k of them, 180 pixels wide at 1024x1024, take 10.3 ms, 6.7 with 16x16.
-// The threshold of the large list stays at the same number of pixels.
+// with 16x16 tiles: another one only where sweeps over triangles from 3 pixels
+// to a third of the image wide lost next to nothing. The numbers of tiles and
+// triangles tell little else: a dense mesh of small triangles and a scene of
+// wide ones, which every tile of the image looks at, count alike.
+//
+// Up to 512 tiles most of the 1216 resident blocks are idle, and where each tile
+// has work enough smaller ones spread it. Setup to fine kernel, of the time with
+// 16x16 tiles (16 to 2000 triangles a tile, 1 to 8 layers): 0.30 to 1.01 with
+// 8x8 up to 256 tiles, 0.61 to 1.04 with 16x8 up to 512. Below 16 triangles a
+// tile or 4096 in all the launches are what takes the time (up to 1.36 with
+// 8x8). From 600 tiles on both gain on closed meshes (768x768, 100k triangles:
+// 61 us with 16x8, 83) and lose elsewhere: 8x8 up to 1.29 at 4 x 256x256, 16x8
+// up to 1.13 there, and 1.39 on 80k triangles 180 pixels wide at 1024x1024. The
+// threshold of the large list stays the same number of tiles: a fourfold one
+// gained up to a third on triangles of 32 to 64 pixels, for four times the
+// bins' memory.
+//
 // Many tiles with few triangles each are bound by the cost per tile: the
-// 64-mesh ragged batch (111k tiles) takes 1002 us with 32x16, 1165 with 16x16;
-// with more than 24 triangles a tile 32x16 is no better (terrain 789, 761). An
-// image whose tiles hold more than 1/912 of all the triangles each (about a
-// block's share) then sets the time: one with 1531 a tile among 979k took
-// 805 us with 32x16, 514 with 16x16. Above four layers the keys of a 32x16
-// tile cost more blocks per SM than it gains (eight: 744, 612 on a sphere). Rows that do
-// not start on 32 bytes leave partial sectors at both ends, half as many with
-// tiles twice as wide (terrain at 2047 pixels: 840 with 32x8, 876).
+// 64-mesh ragged batch (111k tiles) takes 1002 us with 32x16, 1165 with 16x16,
+// 2048x2048 images of triangles 11 to 220 pixels wide 0.50 to 1.03 of 16x16's
+// time, smaller images up to 1.07. With more than 24 triangles a tile 32x16 is
+// no better (terrain 789, 761). An image whose tiles hold more than 1/912 of
+// all the triangles each (about a block's share) then sets the time: one with
+// 1531 a tile among 979k took 805 us with 32x16, 514 with 16x16. Above four
+// layers the keys of a 32x16 tile cost more blocks per SM than it gains (eight:
+// 744, 612 on a sphere). It loses too where hundreds of triangles 600 pixels
+// wide lie over each other (up to 1.18 at 2048x2048). 32x8 for rows that do not
+// start on 32 bytes gained 3 to 8% on small triangles and lost up to 28% on
+// wider ones.
 void default_tile(const Batch& b, int L, int& TW, int& TH) {
   const int64_t tiles = b.tile_start[b.n], tris = b.tri_start[b.n];
   TW = TH = kDefaultTile;
-  if (tiles <= 512 || (tiles <= 1536 && tris >= 16 * tiles)) {
-    TW = TH = 8;
-  } else if (tiles <= 6144 && tris >= 16 * tiles) {
+  if (tiles <= 512 && tris >= std::max(int64_t(4096), 16 * tiles)) {
+    TW = tiles <= 256 ? 8 : 16;
     TH = 8;
-  } else if (tiles >= 16384) {
+  } else if (tiles >= 16384 && L <= 4 && tris <= 24 * tiles) {
     bool even = true;
-    int64_t unaligned = 0;
     for (int i = 0; i < b.n; ++i) {
       const int64_t t = b.tile_start[i + 1] - b.tile_start[i];
       if (912 * (b.tri_start[i + 1] - b.tri_start[i]) > tris * t) even = false;
-      if (b.width[i] % 8 != 0) unaligned += t;
     }
-    if (L <= 4 && tris <= 24 * tiles && even) {
-      TW = 32;
-    } else if (2 * unaligned > tiles) {
-      TW = 32;
-      TH = 8;
-    }
+    if (even) TW = 32;
   }
 }
 
@@ -1080,8 +1083,9 @@ int bounded_large(int large, int64_t tris) {
 }
 
 // The batch table of one group with its tiles, and the workspace it needs.
-// With a tile by the rule that workspace may exceed the 16x16 one, which is
-// then enough too (at 16x16): `min_bytes` is what a call must bring.
+// With a tile by the rule that workspace may exceed the 16x16 one (by its
+// tiles' counts), which is then enough too (at 16x16): `min_bytes` is what a
+// call must bring.
 bool group_batch(const dr_image_desc* images, int n, const dr_raster_config* cfg, int L,
                  size_t ws_bytes, int& TW, int& TH, int& large, Batch& b, Layout& lay,
                  size_t& min_bytes, std::string& err) {
@@ -1096,15 +1100,10 @@ bool group_batch(const dr_image_desc* images, int n, const dr_raster_config* cfg
   Batch ruled;
   std::string ignored;
   if (!make_batch(images, n, L, w, h, ruled, ignored)) return true;  // too many tiles
-  int ruled_large = large;
-  if (cfg->large_tiles <= 0)
-    ruled_large = std::max(large, large * kDefaultTile * kDefaultTile / (w * h));
-  if (ruled_large != bounded_large(ruled_large, b.tri_start[n])) return true;
-  const Layout l = make_layout(ruled.tri_start[n], ruled.tile_start[n], n, ruled_large);
+  const Layout l = make_layout(ruled.tri_start[n], ruled.tile_start[n], n, large);
   if (l.total > ws_bytes) return true;
   b = ruled;
   lay = l;
-  large = ruled_large;
   TW = w;
   TH = h;
   return true;

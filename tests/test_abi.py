@@ -95,6 +95,30 @@ def test_bins_fit_32_bits(tris, w, h):
       assert bins < (1 << 31) + 64  # 256 bytes of alignment
 
 
+# A smaller default tile shows in the workspace by its tiles' counts (16 bytes
+# each) alone: the triangles' share does not grow with it. It is taken up to 512
+# 16x16 tiles with 16 triangles each and 4096 in all, where it never loses.
+@pytest.mark.parametrize("w,h,tris,layers,smaller", [
+    (64, 64, 4095, 3, 1), (64, 64, 4096, 3, 4), (256, 256, 4096, 3, 4), (256, 256, 4095, 3, 1),
+    (256, 256, 1_000_000, 3, 4), (272, 256, 20_000, 3, 2), (512, 256, 8192, 3, 2),
+    (512, 256, 8191, 3, 1), (512, 256, 40_000_000, 3, 2), (528, 256, 100_000, 3, 1),
+    (512, 512, 20_000, 3, 1), (768, 768, 100_000, 3, 1), (1024, 1024, 80_000, 3, 1),
+    (1283, 717, 100_000, 1, 1), (2047, 2048, 1_000_000, 3, 1), (2047, 2048, 1000, 5, 1)])
+def test_default_tile_and_its_workspace(w, h, tris, layers, smaller):
+  lib = _lib.load()
+  b = kernels.ImageBatch.single(w, h, 3, tris)
+
+  def need(tile):
+    cfg = kernels.raster_config(layers, 1, 0, tile)
+    return lib.dr_rasterize_batch_workspace_bytes(b.ptr, 1, ctypes.byref(cfg))
+  tiles = ((w + 15) // 16) * ((h + 15) // 16)
+  extra = need((0, 0)) - need((16, 16))
+  if smaller == 1:
+    assert extra == 0
+  else:
+    assert 0 < extra <= 16 * ((smaller - 1) * tiles + 2 * (w + h)) + 4 * 256
+
+
 def test_entry_points_reject_bad_arguments_without_gpu_work():
   lib = _lib.load()
   b = kernels.ImageBatch.single(8, 8, 3, 1)
