@@ -103,20 +103,27 @@ def _p(t):
   return None if t is None else t.data_ptr()
 
 
-def _stream(device=None):
-  """Handle of the current stream of a device (None: the current one). Every
-  op asks for it before its call, so this is where host tensors are refused
-  that no check before it caught."""
-  index = None
+def _cuda_index(device):
+  """Ordinal of a CUDA device in any of its forms (None: the current one)."""
   if device is not None:
     if not isinstance(device, torch.device):
       device = torch.device(device)
     if device.type != "cuda":
       raise ValueError("diffren_gb300 ops take CUDA tensors; got a %s device" % device)
-    index = device.index
-  if index is None:
-    index = torch.cuda.current_device()
-  return torch._C._cuda_getCurrentRawStream(index)
+    if device.index is not None:
+      return device.index
+  return torch.cuda.current_device()
+
+
+_DEVICE = torch.device
+
+
+def _stream(device=None):
+  """Handle of the current stream of a device (None: the current one). Every
+  op asks for it before its call, so this is where host tensors are refused
+  that no check before it caught (their devices have no index)."""
+  index = device.index if device.__class__ is _DEVICE else None
+  return torch._C._cuda_getCurrentRawStream(_cuda_index(device) if index is None else index)
 
 
 def _f32(t, device=None):
