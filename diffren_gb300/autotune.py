@@ -10,10 +10,13 @@ per-pixel exact), so tuning only changes speed.
 
 ``tune`` times each candidate on the caller's actual inputs with CUDA events
 and keeps the fastest; results are cached in memory and in a JSON file keyed
-by the device, the layer count, the culling and depth modes, the attribute
-width and the batch's size class (image count, log2 of pixels and of
-triangles), so a later process with a similar batch skips the search.
+by the device, the kernels (a digest of the library), the layer count, the
+culling and depth modes, the attribute width and the batch's size class (image
+count, log2 of pixels and of triangles), so a later process with a similar batch
+skips the search, and one with other kernels times its own.
 """
+import functools
+import hashlib
 import json
 import math
 import os
@@ -24,7 +27,8 @@ import torch
 from . import _lib
 from . import kernels
 
-# (tile_width, tile_height, large_tiles); tile_width * tile_height <= 1024.
+# (tile_width, tile_height, large_tiles); tile_width * tile_height <= 1024. Every
+# tile that the rasterizer takes by itself where none is given is among them.
 CANDIDATES = [
     (16, 16, 16), (16, 16, 8), (16, 16, 32),
     (32, 16, 16), (16, 8, 16), (32, 32, 16), (8, 8, 16), (32, 8, 16),
@@ -43,13 +47,23 @@ def cache_path():
   return os.path.join(root, "diffren_gb300", "autotune.json")
 
 
+@functools.lru_cache(maxsize=None)
+def kernels_digest(path=None):
+  """Digest of the library that a choice was timed with."""
+  path = path or _lib.library_path()
+  if not os.path.exists(path):
+    _lib.load()  # builds it
+  with open(path, "rb") as f:
+    return hashlib.sha256(f.read()).hexdigest()[:12]
+
+
 def signature(device_name, batch, config, channels):
-  """Cache key: device, layers, culling, depth mode, attribute width and the
-  batch's size class."""
+  """Cache key: device, kernels, layers, culling, depth mode, attribute width
+  and the batch's size class."""
   px = max(1, batch.total_pixels)
   tris = max(1, batch.total_triangles)
-  return "%s|L%d|c%d|d%d|k%d|n%d|p%d|t%d" % (
-      device_name, config.num_layers, config.face_culling_mode, config.depth_mode,
+  return "%s|%s|L%d|c%d|d%d|k%d|n%d|p%d|t%d" % (
+      device_name, kernels_digest(), config.num_layers, config.face_culling_mode, config.depth_mode,
       int(channels), batch.n, round(math.log2(px)), round(math.log2(tris)))
 
 

@@ -68,3 +68,43 @@ def test_time_candidates_picks_fastest_and_skips_rejected():
 def test_candidates_fit_the_rasterizer_limits():
   for w, h, large in autotune.CANDIDATES:
     assert 0 < w <= 128 and 0 < h <= 128 and w * h <= 1024 and large > 0
+
+
+def test_choices_of_other_kernels_are_not_found(tmp_path, monkeypatch):
+  b, c = batch_and_config()
+  path = str(tmp_path / "tune.json")
+  keys = []
+  for k in range(2):
+    lib = tmp_path / ("lib%d.so" % k)
+    lib.write_bytes(b"kernels %d" % k)
+    monkeypatch.setenv("DIFFREN_GB300_LIBRARY", str(lib))
+    autotune.kernels_digest.cache_clear()
+    keys.append(autotune.signature("GB300", b, c, 4))
+  autotune.kernels_digest.cache_clear()
+  autotune.clear_memory()
+  autotune.store(keys[0], (8, 8, 16), path)
+  autotune.clear_memory()
+  assert autotune.lookup(keys[0], path) == (8, 8, 16)
+  assert autotune.lookup(keys[1], path) is None
+  autotune.clear_memory()
+
+
+def test_default_tiles_are_candidates():
+  """The tile that no configuration gives shows in the workspace it needs
+  (which also covers 16x16): it is that of a candidate with 16 tiles as the
+  large threshold, as in the default."""
+  chosen = set()
+  for w, h, images, tris, layers in (
+      (64, 64, 1, 5000, 3), (256, 256, 1, 300, 3), (256, 256, 1, 20000, 1), (352, 340, 1, 20000, 3),
+      (640, 480, 1, 20000, 4), (1024, 1024, 8, 100000, 3), (1000, 1000, 64, 20000, 3),
+      (1000, 1000, 64, 20000, 8), (2047, 2047, 4, 1000000, 3)):
+    batch = kernels.ImageBatch([w] * images, [h] * images, [3] * images, [tris] * images)
+
+    def need(tile, large):
+      return kernels.raster_workspace_bytes(batch, kernels.raster_config(layers, 1, 0, tile, large))
+    base = need((16, 16), 16)
+    fits = {c for c in autotune.CANDIDATES
+            if c[2] == 16 and max(base, need(c[:2], 16)) == need((0, 0), 0)}
+    assert fits
+    chosen |= fits
+  assert {(16, 16, 16), (8, 8, 16), (16, 8, 16)} <= chosen
