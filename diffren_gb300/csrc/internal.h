@@ -59,6 +59,10 @@ inline bool make_batch(const dr_image_desc* images, int n, int L, int TW, int TH
 
 constexpr int kMaxDevices = 64;
 
+// SMs of a GB300, in the rules that split work by how many blocks run at once:
+// they were measured on it, and the workspace query follows one without a device.
+constexpr int kSms = 152;
+
 // Host-side cache of one kernel's launch attributes on each device: the
 // dynamic shared-memory limit raised so far, and SMs x resident blocks per
 // SM for the last few shared-memory sizes. Host threads may launch

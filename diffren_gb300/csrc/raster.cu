@@ -449,7 +449,7 @@ constexpr int kPush = 8, kQueue = 32 * kPush + 32;
 // blocks of 128 fit an SM's shared memory, as the registers allow, and every
 // further chunk costs: the fine kernel takes 545 us on the 4 x 2048^2 terrain
 // with 128, 574 with 96, 625 with 64. Above, 64 keep eight blocks up to eight
-// layers of 16x16, where 128 leave seven to five: 800 us on the 64-mesh
+// layers of 16x16, where 128 leave seven or six: 800 us on the 64-mesh
 // ragged batch in 32x16 tiles (883 with 128); setup to fine kernel for a
 // 100k-triangle sphere (8 x 1024^2) 454 us (466) at four layers, 535 (579) at
 // six, 612 (649) at eight.
@@ -1033,7 +1033,7 @@ bool check_config(const dr_raster_config* cfg, int& L, int& TW, int& TH, int& la
 // triangles tell little else: a dense mesh of small triangles and a scene of
 // wide ones, which every tile of the image looks at, count alike.
 //
-// Up to 512 tiles most of the 1216 resident blocks are idle, and where each tile
+// Up to 512 tiles most of the resident blocks (eight on each SM) are idle, and where each tile
 // has work enough smaller ones spread it. Setup to fine kernel, of the time with
 // 16x16 tiles (16 to 2000 triangles a tile, 1 to 8 layers): 0.30 to 1.01 with
 // 8x8 up to 256 tiles, 0.61 to 1.04 with 16x8 up to 512. Below 16 triangles a
@@ -1049,7 +1049,7 @@ bool check_config(const dr_raster_config* cfg, int& L, int& TW, int& TH, int& la
 // 64-mesh ragged batch (111k tiles) takes 1002 us with 32x16, 1165 with 16x16,
 // 2048x2048 images of triangles 11 to 220 pixels wide 0.50 to 1.03 of 16x16's
 // time, smaller images up to 1.07. With more than 24 triangles a tile 32x16 is
-// no better (terrain 789, 761). An image whose tiles hold more than 1/912 of
+// no better (terrain 789, 761). An image whose tiles hold more than a 912th of
 // all the triangles each (about a block's share) then sets the time: one with
 // 1531 a tile among 979k took 805 us with 32x16, 514 with 16x16. Above four
 // layers the keys of a 32x16 tile cost more blocks per SM than it gains (eight:
@@ -1067,7 +1067,7 @@ void default_tile(const Batch& b, int L, int& TW, int& TH) {
     bool even = true;
     for (int i = 0; i < b.n; ++i) {
       const int64_t t = b.tile_start[i + 1] - b.tile_start[i];
-      if (912 * (b.tri_start[i + 1] - b.tri_start[i]) > tris * t) even = false;
+      if (6 * kSms * (b.tri_start[i + 1] - b.tri_start[i]) > tris * t) even = false;
     }
     if (even) TW = 32;
   }

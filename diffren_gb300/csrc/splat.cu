@@ -262,8 +262,7 @@ __device__ __forceinline__ void scatter_runs(const SampleArgs& a, const PosArgs&
                                              const Batch& B, int lane, int last, bool leader,
                                              bool on, int im, int64_t el, const float (&b)[3],
                                              const int (&vid)[3], const float4 (&V)[3],
-                                             float4 dcl, float (&db)[3], float& mx,
-                                             int scale) {
+                                             float4 dcl, float (&db)[3], int scale) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const float bi = b[i];
@@ -405,7 +404,6 @@ __global__ void __launch_bounds__(kVjpThreads, 6) samples_bwd_kernel(SampleArgs 
     const bool on = k < n;
     int im = 0;
     const int64_t el = on ? element(s_list[k], im) : 0;
-    int id = -1;
     float b[3] = {0.0f, 0.0f, 0.0f};
     int vid[3] = {0, 0, 0};
     float4 V[3] = {make_float4(0.0f, 0.0f, 0.0f, 1.0f), make_float4(0.0f, 0.0f, 0.0f, 1.0f),
@@ -420,10 +418,8 @@ __global__ void __launch_bounds__(kVjpThreads, 6) samples_bwd_kernel(SampleArgs 
         // Vertex indices stored by the rasterizer: no triangle gather.
 #pragma unroll
         for (int i = 0; i < 3; ++i) vid[i] = __ldg(a.vid + 3 * el + i);
-        id = vid[0];
       } else {
-        id = __ldg(p.ids + el);
-        const int32_t* t = p.tris + 3 * (B.triangle_offset[im] + id);
+        const int32_t* t = p.tris + 3 * (B.triangle_offset[im] + __ldg(p.ids + el));
 #pragma unroll
         for (int i = 0; i < 3; ++i) vid[i] = __ldg(t + i);
       }
@@ -476,7 +472,6 @@ __global__ void __launch_bounds__(kVjpThreads, 6) samples_bwd_kernel(SampleArgs 
     const int p_v1 = __shfl_up_sync(0xffffffffu, vid[1], 1);
     const int p_v2 = __shfl_up_sync(0xffffffffu, vid[2], 1);
     const bool differs = (kim != p_im) | (vid[0] != p_v0) | (vid[1] != p_v1) | (vid[2] != p_v2);
-    (void)id;
     const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || differs);
     const unsigned later = heads & ~((2u << lane) - 1u);  // heads after this lane
     const int last = later ? __ffs(later) - 2 : 31;
@@ -485,19 +480,19 @@ __global__ void __launch_bounds__(kVjpThreads, 6) samples_bwd_kernel(SampleArgs 
     const unsigned span = __reduce_max_sync(0xffffffffu, unsigned(last - lane));
     float db[3];
     if (span == 0)
-      scatter_runs<0, kMode>(a, p, B, lane, last, leader, on, im, el, b, vid, V, dcl, db, mx,
+      scatter_runs<0, kMode>(a, p, B, lane, last, leader, on, im, el, b, vid, V, dcl, db,
                              scale);
     else if (span < 2)
-      scatter_runs<1, kMode>(a, p, B, lane, last, leader, on, im, el, b, vid, V, dcl, db, mx,
+      scatter_runs<1, kMode>(a, p, B, lane, last, leader, on, im, el, b, vid, V, dcl, db,
                              scale);
     else if (span < 4)
-      scatter_runs<2, kMode>(a, p, B, lane, last, leader, on, im, el, b, vid, V, dcl, db, mx,
+      scatter_runs<2, kMode>(a, p, B, lane, last, leader, on, im, el, b, vid, V, dcl, db,
                              scale);
     else if (span < 8)
-      scatter_runs<3, kMode>(a, p, B, lane, last, leader, on, im, el, b, vid, V, dcl, db, mx,
+      scatter_runs<3, kMode>(a, p, B, lane, last, leader, on, im, el, b, vid, V, dcl, db,
                              scale);
     else
-      scatter_runs<5, kMode>(a, p, B, lane, last, leader, on, im, el, b, vid, V, dcl, db, mx,
+      scatter_runs<5, kMode>(a, p, B, lane, last, leader, on, im, el, b, vid, V, dcl, db,
                              scale);
     if (on && p.d_bary) {
       p.d_bary[3 * el] = db[0];
@@ -1867,10 +1862,10 @@ int samples_bwd_launch(const float* d_attr_out, const float* d_positions,
       if (!make_batch(images + g0, cnt, L, kTX, kTY, b, err)) return DR_ERR_INVALID_ARGUMENT;
       const int64_t total = int64_t(L) * b.pix_prefix[cnt];
       if (total <= 0) continue;
-      // Below two waves of full blocks (six on each of 152 SMs), one sample a
-      // thread: small images otherwise leave most SMs idle (196k samples in 48
-      // blocks took 26 us, in 768 blocks 8).
-      const bool few = total < int64_t(2) * 912 * kVjpThreads * kVjpPer;
+      // Below two waves of full blocks (six on each SM), one sample a thread:
+      // small images otherwise leave most SMs idle (196k samples in 48 blocks
+      // took 26 us, in 768 blocks 8).
+      const bool few = total < int64_t(2) * 6 * kSms * kVjpThreads * kVjpPer;
       const int64_t block = int64_t(kVjpThreads) * (few ? 1 : kVjpPer);
       const unsigned grid = unsigned((total + block - 1) / block);
       using Kernel = void (*)(SampleArgs, Batch);

@@ -498,7 +498,7 @@ int dr_vertex_normals_csr_bwd(const float* d_normals, const float* vertices,
  * foreground flag. colors [L, H, W, C]
  * (1 <= C <= DR_MAX_SPLAT_CHANNELS, last channel alpha); out [H, W, C].
  * saved [3 (C + 1) + 2, P] receives the fg/surface/bg accumulators and
- * weights the VJP needs and (for three layers) each pixel's surface classes
+ * weights the VJP needs and (for two and three layers) each pixel's surface classes
  * of its 9 taps as a 32-bit code, P = the largest pixel_offset + width *
  * height of the images, then the list of the screen tiles that hold
  * foreground: one plane of P pixels per value, or, for four channels in a
