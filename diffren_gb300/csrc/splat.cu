@@ -248,7 +248,6 @@ __device__ __forceinline__ float4 run_sum4(float4 v, int lane, int last) {
 }
 
 constexpr int kVjpThreads = 256;
-constexpr int kVjpPer = 8;  // samples whose depth each thread tests
 
 // The run-summed scatter of one compacted foreground sample per lane into
 // the vertex gradients (clip and attributes) and its barycentric adjoint
@@ -325,9 +324,12 @@ __device__ __forceinline__ void scatter_runs(const SampleArgs& a, const PosArgs&
 // (same-address atomics serialize in L2). Six blocks of 256 threads per SM,
 // each warp reading whole lines: 394 us on the 64-mesh ragged batch (85 M
 // samples, 9.2 M foreground) where a block-wide scan over eight consecutive
-// samples a thread took 512; 146 us (180) on the 8 x 1024^2 sphere.
+// samples a thread took 512; 146 us (180) on the 8 x 1024^2 sphere. The fixed-
+// point passes wait on more and longer atomics and take eight blocks: 315 us on
+// 4 x 1000^2 soups of three layers, 369 with six.
 template <int kMode, int kPer>
-__global__ void __launch_bounds__(kVjpThreads, 6) samples_bwd_kernel(SampleArgs a, Batch B) {
+__global__ void __launch_bounds__(kVjpThreads, kMode == 0 ? 6 : 8)
+    samples_bwd_kernel(SampleArgs a, Batch B) {
   constexpr int kBlock = kVjpThreads * kPer, kWarps = kVjpThreads / 32;
   __shared__ unsigned short s_list[kBlock];  // sample - the block's first
   __shared__ int s_count[kWarps];
@@ -1862,18 +1864,21 @@ int samples_bwd_launch(const float* d_attr_out, const float* d_positions,
       if (!make_batch(images + g0, cnt, L, kTX, kTY, b, err)) return DR_ERR_INVALID_ARGUMENT;
       const int64_t total = int64_t(L) * b.pix_prefix[cnt];
       if (total <= 0) continue;
-      // Below two waves of full blocks (six on each SM), one sample a thread:
-      // small images otherwise leave most SMs idle (196k samples in 48 blocks
-      // took 26 us, in 768 blocks 8).
-      const bool few = total < int64_t(2) * 6 * kSms * kVjpThreads * kVjpPer;
-      const int64_t block = int64_t(kVjpThreads) * (few ? 1 : kVjpPer);
+      // Samples a thread: one where the blocks are two per place on the device
+      // or fewer (small images otherwise leave most SMs idle: 196k samples take
+      // 8 us, 26 with eight), then four up to six (16 in fixed point) of them,
+      // then eight, as a block's list costs what it costs: 1 M dense samples 18
+      // us with four, 27 with one, 22 with eight; 3 M 51, 32 and 30.
+      const int64_t full = int64_t(6) * kSms * kVjpThreads;
+      const int size = total < 2 * full ? 0 : total < (mode == 0 ? 6 : 16) * full ? 1 : 2;
+      const int64_t block = int64_t(kVjpThreads) * (size == 0 ? 1 : size == 1 ? 4 : 8);
       const unsigned grid = unsigned((total + block - 1) / block);
       using Kernel = void (*)(SampleArgs, Batch);
-      const Kernel kernels[2][3] = {
-          {samples_bwd_kernel<0, kVjpPer>, samples_bwd_kernel<1, kVjpPer>,
-           samples_bwd_kernel<2, kVjpPer>},
-          {samples_bwd_kernel<0, 1>, samples_bwd_kernel<1, 1>, samples_bwd_kernel<2, 1>}};
-      kernels[few][mode]<<<grid, kVjpThreads, 0, stream>>>(am, b);
+      const Kernel kernels[3][3] = {
+          {samples_bwd_kernel<0, 1>, samples_bwd_kernel<1, 1>, samples_bwd_kernel<2, 1>},
+          {samples_bwd_kernel<0, 4>, samples_bwd_kernel<1, 4>, samples_bwd_kernel<2, 4>},
+          {samples_bwd_kernel<0, 8>, samples_bwd_kernel<1, 8>, samples_bwd_kernel<2, 8>}};
+      kernels[size][mode]<<<grid, kVjpThreads, 0, stream>>>(am, b);
     }
   }
   if (det && nv > 0)

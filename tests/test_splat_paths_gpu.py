@@ -95,6 +95,16 @@ def test_samples_vjp_block_rule(sizes, layers, channels, deterministic, device):
     assert (x.double() - y).abs().max() <= 1e-4 * y.abs().max()
 
 
+# Four samples a thread from 467k samples on, to 1.4 M, or 3.7 M in fixed point;
+# the first two sizes lie on both sides of the lower line.
+@pytest.mark.parametrize("sizes,layers,channels", [
+    ([(683, 683)], 1, 4), ([(684, 684)], 1, 4), ([(97, 131)] * 40 + [(3, 1)] * 9, 2, 3),
+    ([(1183, 1184)], 1, 2), ([(1184, 1184)], 1, 2), ([(640, 480), (901, 703)], 3, 9)])
+@pytest.mark.parametrize("deterministic", [False, True])
+def test_samples_vjp_four_a_thread(sizes, layers, channels, deterministic, device):
+  test_samples_vjp_block_rule(sizes, layers, channels, deterministic, device)
+
+
 # Four channels in a 16-byte aligned buffer save float4 planes, anything else
 # one plane per value; both hold the same numbers.
 @pytest.mark.parametrize("layers", [1, 2, 3])
