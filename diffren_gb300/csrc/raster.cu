@@ -444,6 +444,9 @@ struct FineSmem {
 // A row pushes up to kPush candidates at a time; fewer than 32 are carried
 // from one push to the next.
 constexpr int kPush = 8, kQueue = 32 * kPush + 32;
+// Between chunks the queues hold gather_large's list.
+static_assert(kThreads / 32 * kQueue * sizeof(unsigned short) >= kThreads * sizeof(int),
+              "gather_large's list");
 
 // Triangles a chunk holds. Up to 768 keys (16x16 pixels of three layers) eight
 // blocks of 128 fit an SM's shared memory, as the registers allow, and every
@@ -672,6 +675,60 @@ __device__ __forceinline__ void fill_background(const RasterArgs& a, const TileB
   if (kFused && a.so.attr && !a.fg_attr) fill_rows(a.so.attr_out, a.so.K, 0.0f, t, L);
 }
 
+// The next chunk of a tile whose image has more large triangles than a chunk
+// holds: the nrest < kChunk triangles that its bins still have (none where
+// negative), then those of the large list whose box meets the tile's. Taken as
+// they lie, most chunks of such a list hold a handful of triangles for this
+// tile, and a chunk costs its chain of loads and barriers whatever it holds:
+// 100k triangles 110 pixels wide at 1024x1024 took 4.57 ms (3.41 before a
+// chunk's rows were narrowed and queued), with full chunks 2.35. Boxes are
+// looked at 128 at a time, four groups of loads in flight. list: kChunk
+// integers. scan: the first triangle of the next group, and how many of that
+// group's hits an earlier chunk took.
+template <int kChunk>
+__device__ __forceinline__ int gather_large(const int32_t* large, int nlarge, const uint2* boxes,
+                                            const int32_t* rest, int nrest, int4 tile, int* list,
+                                            int* s_warp, int2* scan) {
+  const int tid = threadIdx.x;
+  int next = scan->x, skip = scan->y;
+  int have = max(0, nrest);
+  if (tid < have) list[tid] = rest[tid];
+  while (have < kChunk && next < nlarge) {
+    constexpr int kAhead = 4;
+    int g[kAhead];
+    uint2 box[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const int i = next + k * kThreads + tid;
+      g[k] = i < nlarge ? large[i] : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) box[k] = g[k] >= 0 ? boxes[g[k]] : make_uint2(0u, 0u);
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      if (have >= kChunk) break;
+      const int4 b = unpack_box(box[k]);
+      const bool hit = b.y > tile.x && b.x < tile.y && b.w > tile.z && b.z < tile.w;
+      int rank;
+      const int all = block_exclusive_scan<kThreads>(hit ? 1 : 0, s_warp, rank) - skip;
+      const int at = have + rank - skip;
+      if (hit && at >= have && at < kChunk) list[at] = g[k];
+      if (all > kChunk - have) {  // the rest of this group is the next chunk's
+        skip += kChunk - have;
+        have = kChunk;
+      } else {
+        have += all;
+        skip = 0;
+        next += kThreads;
+      }
+    }
+  }
+  __syncthreads();
+  if (tid == 0) *scan = make_int2(next, skip);
+  __syncthreads();
+  return tid < have ? list[tid] : -1;
+}
+
 // Persistent fine rasterizer. Each block takes (image, tile) items from a
 // global queue (heaviest tiles first, in tile_order_kernel's order), keeps
 // the tile's L x TW x TH packed keys in shared memory, and spreads the rows
@@ -692,6 +749,7 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a, 
   __shared__ int s_warp[kThreads / 32];
   __shared__ QueueItem s_item;
   __shared__ int s_nfg;
+  __shared__ int2 s_scan;  // where the scan of the image's large list stands
   const int TW = a.TW, TH = a.TH, TP = TW * TH, L = LT > 0 ? LT : a.L;
   FineSmem s;
   {
@@ -738,7 +796,8 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a, 
     }
     const int bin0 = tb.bin0, nbin = tb.nbin;
     const int nlarge = a.large_count[img];
-    const int nsrc = nbin + nlarge;
+    int nsrc = nbin + nlarge;
+    if (threadIdx.x == 0) s_scan = make_int2(0, 0);
     // Fixed-point x to pixel index: x = px W / 131072 + W / 2 - 1/2. Rounding
     // the pixel centers to fixed point moves them by at most 2 units, and
     // the float32 steps here stay below 0.02 pixels.
@@ -749,9 +808,16 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a, 
 
     for (int c0 = 0; c0 < nsrc; c0 += kChunk) {
       const int i = c0 + threadIdx.x;
-      int cnt = 0, g = 0, cx0 = 0, cy0 = 0, cw = 1;
-      if ((kChunk == kThreads || threadIdx.x < kChunk) && i < nsrc) {
+      int cnt = 0, g = -1, cx0 = 0, cy0 = 0, cw = 1;
+      if (nlarge > kChunk && c0 + kChunk > nbin) {
+        g = gather_large<kChunk>(a.large_list + tri0, nlarge, a.box, a.bins + bin0 + c0, nbin - c0,
+                                 make_int4(x0, x0 + tw, y0, y0 + th),
+                                 reinterpret_cast<int*>(s.queue), s_warp, &s_scan);
+        if (s_scan.x >= nlarge) nsrc = 0;  // the last chunk
+      } else if ((kChunk == kThreads || threadIdx.x < kChunk) && i < nsrc) {
         g = i < nbin ? a.bins[bin0 + i] : a.large_list[tri0 + (i - nbin)];
+      }
+      if (g >= 0) {
         const int4 box = unpack_box(a.box[g]);
         cx0 = max(box.x, x0) - x0;
         cy0 = max(box.z, y0) - y0;

@@ -117,3 +117,39 @@ def test_chunk_of_large_tiles(count, layers, device):
     for got in out[k + 1:k + 5]:
       for a, b in zip(got, out[k]):
         assert torch.equal(a, b)
+
+
+# An image with more large triangles than a chunk holds (128, or 64 above 768 keys
+# a tile) has its chunks gathered from the list 128 boxes at a time, after the
+# bins' last ones: a threshold of 1 tile (nearly all are large), one in between,
+# and one that leaves the list empty give the same bits, as does the oracle.
+@pytest.mark.parametrize("wide,small", [(63, 5), (65, 0), (127, 1), (128, 200), (129, 0), (255, 130),
+                                        (257, 7), (512, 64), (513, 0), (900, 900)])
+@pytest.mark.parametrize("layers,tile", [(3, (16, 16)), (1, (8, 8)), (5, (16, 16)), (3, (32, 16))])
+def test_large_list_is_gathered(wide, small, layers, tile, device):
+  w, h = 150, 90
+  rng = np.random.default_rng(wide)
+  center = rng.uniform(-1, 1, (wide + small, 1, 3))
+  reach = np.where(np.arange(wide + small) < wide, 0.7, 0.02)[:, None, None]
+  verts = (center + reach * rng.uniform(-1, 1, (wide + small, 3, 3))).reshape(-1, 3)
+  order = rng.permutation(wide + small)
+  clip = np.concatenate([verts, np.ones((len(verts), 1))], 1).astype(np.float32)
+  tri = np.arange(len(verts), dtype=np.int32).reshape(-1, 3)[order]
+  dclip, dtri = torch.tensor(clip, device=device), torch.tensor(tri, device=device)
+  # a second image with an empty list, and a third like the first
+  tiny = dclip[:3] * torch.tensor([0.05, 0.05, 1.0, 1.0], device=device)
+  batch = kernels.ImageBatch([w, 40, w], [h, 30, h], [len(clip), 3, len(clip)],
+                             [len(tri), 1, len(tri)])
+  clips = torch.cat([dclip, tiny, dclip])
+  tris = torch.cat([dtri, torch.arange(3, dtype=torch.int32, device=device)[None], dtri])
+  out = [kernels.rasterize_packed(clips, tris, batch, kernels.raster_config(
+      layers, 0, _lib.DR_DEPTH_DISCRETIZED, tile, large)) for large in (100000, 1, 6)]
+  for got in out[1:]:
+    for a, b in zip(got, out[0]):
+      assert torch.equal(a, b)
+  n = layers * w * h
+  ref = raster.rasterize(clip, tri, w, h, layers, 0, raster.DEPTH_DISCRETIZED)
+  for part in (slice(0, n), slice(out[1][0].numel() - n, None)):
+    ids, z, bary = (x[part].cpu().numpy() for x in out[1])
+    assert_same((ids.reshape(layers, h, w), z.reshape(layers, h, w),
+                 bary.reshape(layers, h, w, 3)), ref)
