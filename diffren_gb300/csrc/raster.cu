@@ -586,32 +586,37 @@ __device__ __forceinline__ TileBox tile_box(const RasterArgs& a, const Batch& B,
 }
 
 // The fine rasterizer's queue: the occupied tiles in order, then the empty
-// ones kEmptyRun at a time (they only write background samples).
-constexpr int kEmptyRun = 8;
+// ones in runs (they only write background samples). A run is as long as two
+// for every block allow, up to kEmptyRun: always eight left most blocks without
+// work in images of a few thousand tiles (1024x1024, eight layers, 300 tiny
+// triangles: 58 us, 43 so).
+constexpr unsigned kEmptyRun = 8;
 
 struct Queue {
-  unsigned occupied, items;
+  unsigned occupied, items, run;
 };
 
 __device__ __forceinline__ Queue make_queue(const RasterArgs& a) {
   const unsigned empty = a.counters[2 + kEmptyClass];
   Queue q;
   q.occupied = unsigned(a.total_tiles) - empty;
-  q.items = q.occupied + (empty + kEmptyRun - 1) / kEmptyRun;
+  q.run = min(max(empty / (2 * gridDim.x), 1u), kEmptyRun);
+  q.items = q.occupied + (empty + q.run - 1) / q.run;
   return q;
 }
 
 // One item as its block sees it.
 struct QueueItem {
   int kind;  // 0 tile, 1 empty run, 2 end
-  uint3 o;   // tile: its words; run: o.x = its first entry
+  uint3 o;   // tile: its words; run: its first entry and the one after its last
 };
 
 __device__ __forceinline__ QueueItem queue_item(const RasterArgs& a, const Queue& q,
                                                 unsigned head) {
   QueueItem it;
   it.kind = head < q.occupied ? 0 : head < q.items ? 1 : 2;
-  it.o = make_uint3(q.occupied + (head - q.occupied) * kEmptyRun, 0u, 0u);
+  const unsigned first = q.occupied + (head - q.occupied) * q.run;
+  it.o = make_uint3(first, min(first + q.run, unsigned(a.total_tiles)), 0u);
   if (it.kind == 0) it.o = tile_words(a, int(head));
   return it;
 }
@@ -747,6 +752,7 @@ template <bool kFused, int LT, int kChunk>
 __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a, Batch B) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_warp[kThreads / 32];
+  __shared__ Queue s_queue;  // thread 0's: in registers it would take every thread's
   __shared__ QueueItem s_item;
   __shared__ int s_nfg;
   __shared__ int2 s_scan;  // where the scan of the image's large list stands
@@ -771,14 +777,14 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a, 
   const unsigned long long kEmpty = empty_key(a.depth_mode);
   const bool disc = a.depth_mode == DR_DEPTH_DISCRETIZED;
 
-  const Queue queue = make_queue(a);
+  if (threadIdx.x == 0) s_queue = make_queue(a);
   for (;;) {
-    if (threadIdx.x == 0) s_item = queue_item(a, queue, atomicAdd(&a.counters[0], 1u));
+    if (threadIdx.x == 0) s_item = queue_item(a, s_queue, atomicAdd(&a.counters[0], 1u));
     __syncthreads();
     const QueueItem it = s_item;
     if (it.kind == 2) break;
     if (it.kind == 1) {
-      for (int k = int(it.o.x); k < min(int(it.o.x) + kEmptyRun, a.total_tiles); ++k)
+      for (int k = int(it.o.x); k < int(it.o.y); ++k)
         fill_background<kFused>(a, tile_box(a, B, tile_words(a, k), L), L);
       __syncthreads();
       continue;

@@ -153,3 +153,28 @@ def test_large_list_is_gathered(wide, small, layers, tile, device):
     ids, z, bary = (x[part].cpu().numpy() for x in out[1])
     assert_same((ids.reshape(layers, h, w), z.reshape(layers, h, w),
                  bary.reshape(layers, h, w, 3)), ref)
+
+
+# Empty tiles come in runs of one to eight, by their number: the depths of nearly
+# empty images from hundreds to a hundred thousand tiles, and of one with none.
+@pytest.mark.parametrize("w,h", [(260, 250), (1111, 700), (2304, 2200)])
+@pytest.mark.parametrize("tile", [(8, 8), (16, 16), (128, 8)])
+@pytest.mark.parametrize("empty", [False, True])
+def test_empty_runs(w, h, tile, empty, device):
+  clip = torch.tensor([[0.5, 0.5, 0.1, 1.0], [0.9, 0.5, 0.1, 1.0], [0.5, 0.95, 0.1, 1.0]],
+                      device=device)
+  tri = torch.arange(0 if empty else 3, dtype=torch.int32, device=device).view(-1, 3)
+  batch = kernels.ImageBatch.single(w, h, 3, len(tri))
+  out = (torch.full((2 * w * h,), -7, dtype=torch.int32, device=device),
+         torch.full((2 * w * h,), float("nan"), device=device),
+         torch.full((2 * w * h, 3), float("nan"), device=device))
+  ids, z, bary = kernels.rasterize_packed(
+      clip, tri, batch, kernels.raster_config(2, 0, _lib.DR_DEPTH_FLOAT, tile), out=out)
+  z = z.view(2, h, w)
+  covered = z[0] != 1.0
+  assert not torch.isnan(z).any() and not torch.isnan(bary).any() and (z[1] == 1.0).all()
+  assert torch.equal(ids.view(2, h, w)[0], torch.where(covered, 0, -1).int())
+  assert (ids.view(2, h, w)[1] == -1).all() and not bary.view(2, h, w, 3)[1].any()
+  # half of a 0.2 x 0.225 box of the image, within its outline's pixels
+  want = 0 if empty else 0.5 * 0.2 * 0.225 * w * h
+  assert abs(int(covered.sum()) - want) <= (0 if empty else 0.3 * (w + h))
