@@ -178,3 +178,21 @@ def test_empty_runs(w, h, tile, empty, device):
   # half of a 0.2 x 0.225 box of the image, within its outline's pixels
   want = 0 if empty else 0.5 * 0.2 * 0.225 * w * h
   assert abs(int(covered.sum()) - want) <= (0 if empty else 0.3 * (w + h))
+
+
+# A row's keys are permuted within the power of two in the tile's width (up to 16).
+@pytest.mark.parametrize("tile", [(1, 16), (2, 3), (6, 10), (12, 20), (4, 40), (8, 33), (24, 16),
+                                  (20, 9), (48, 16), (128, 8), (3, 128)])
+@pytest.mark.parametrize("layers", [1, 3, 6])
+def test_tile_widths_match_oracle(tile, layers, device):
+  for kind, n in (("big", 40), ("soup", 300)):
+    verts, tris = _scene(kind, n, 131, 77, 5)
+    ref = raster.rasterize(verts, tris, 131, 77, layers, 1, raster.DEPTH_DISCRETIZED)
+    clip = torch.tensor(np.asarray(verts, np.float32), device=device)
+    tri = torch.tensor(np.asarray(tris, np.int32), device=device)
+    batch = kernels.ImageBatch.single(131, 77, len(clip), len(tri))
+    got = kernels.rasterize_packed(clip, tri, batch, kernels.raster_config(
+        layers, 1, _lib.DR_DEPTH_DISCRETIZED, tile))
+    shape = (layers, 77, 131)
+    assert_same((got[0].view(shape).cpu().numpy(), got[1].view(shape).cpu().numpy(),
+                 got[2].view(*shape, 3).cpu().numpy()), ref)
