@@ -148,14 +148,17 @@ __global__ void __launch_bounds__(256) texture_fwd_kernel(TexArgs a) {
 // The common cases on 32-bit texel indices: up to four channels, edge padding,
 // a texture of fewer than 2^29 texels and sides up to 2^24 (fits_foot32), 8-byte
 // aligned uv, and for four channels 16-byte aligned texture and output. Same
-// operations and order as texture_fwd_kernel. Each thread takes two points a block's width apart, so
-// that their coordinate loads, and then their texel loads, are in flight
-// together, and six blocks share an SM: the kernels wait on those loads (the
+// operations and order as texture_fwd_kernel. Each thread takes kPoints points a
+// block's width apart, so that their coordinate loads, and then their texel
+// loads, are in flight together, and six blocks share an SM: the kernels wait on
+// those loads. Two points where one a thread would be more than two waves (the
 // 50 M points of the 4 x 2048^2 terrain, forward and backward, take 76 us less
-// of 615 than with one point a thread; four points need registers that cost
-// more). Three channels: 16 and 48 us for 1.5 M points, 19 and 69 us in the
-// general kernels, whose backward issues three reductions a texel, not two.
-constexpr int kPoints = 2;
+// of 615 than with one; four need registers that cost more); below, a block's
+// own latency is what counts: 1000 points take 2.3 and 5.6 us with one, 2.8 and
+// 6.5 with two, 100k 3.2 and 7.9, 3.8 and 8.6. Three channels: 16 and 48 us for
+// 1.5 M points, 19 and 69 us in the general kernels, whose backward issues three
+// reductions a texel, not two.
+int points_a_thread(int64_t n) { return n > int64_t(2) * 6 * kSms * 256 ? 2 : 1; }
 
 // Padding and texture sizes that foot32's indexes stay inside. axis_of clips the
 // floor index to the size as a float, exact up to 2^24; a longer side's may round
@@ -196,7 +199,7 @@ __device__ __forceinline__ void load_texel(const float* tex, unsigned t, float (
   }
 }
 
-template <int C>
+template <int C, int kPoints>
 __global__ void __launch_bounds__(256, 6) texture_fwd32_kernel(TexArgs a) {
   const int64_t i0 = int64_t(blockIdx.x) * (256 * kPoints) + threadIdx.x;
   float2 uv[kPoints];
@@ -255,7 +258,7 @@ __device__ __forceinline__ void add_texel(float* tex, unsigned t, const float (&
 // The VJP of texture_fwd32_kernel (same conditions; d_out and d_tex 16-byte
 // aligned for four channels, d_tex and d_uv 8-byte aligned). Points with a
 // zero gradient read no coordinates.
-template <int C>
+template <int C, int kPoints>
 __global__ void __launch_bounds__(256, 6) texture_bwd32_kernel(TexArgs a) {
   const int64_t i0 = int64_t(blockIdx.x) * (256 * kPoints) + threadIdx.x;
   float g[kPoints][C];
@@ -453,9 +456,13 @@ int texture_fwd_launch(const float* uv, int64_t n, const float* tex, int H, int 
   if (fits_foot32(H, W, C, flags) && (reinterpret_cast<uintptr_t>(uv) & 7) == 0 &&
       (C != 4 || (wide & 15) == 0)) {
     using Kernel = void (*)(TexArgs);
-    const Kernel kernels[4] = {texture_fwd32_kernel<1>, texture_fwd32_kernel<2>,
-                               texture_fwd32_kernel<3>, texture_fwd32_kernel<4>};
-    kernels[C - 1]<<<unsigned((n + 256 * kPoints - 1) / (256 * kPoints)), 256, 0, stream>>>(a);
+    const Kernel kernels[2][4] = {{texture_fwd32_kernel<1, 1>, texture_fwd32_kernel<2, 1>,
+                                   texture_fwd32_kernel<3, 1>, texture_fwd32_kernel<4, 1>},
+                                  {texture_fwd32_kernel<1, 2>, texture_fwd32_kernel<2, 2>,
+                                   texture_fwd32_kernel<3, 2>, texture_fwd32_kernel<4, 2>}};
+    const int points = points_a_thread(n);
+    kernels[points - 1][C - 1]<<<unsigned((n + 256 * points - 1) / (256 * points)), 256, 0,
+                                 stream>>>(a);
   } else {
     texture_fwd_kernel<<<unsigned((n + 255) / 256), 256, 0, stream>>>(a);
   }
@@ -509,9 +516,13 @@ int texture_bwd_launch(const float* d_out, const float* uv, int64_t n, const flo
                          reinterpret_cast<uintptr_t>(d_tex);
   if (fits_foot32(H, W, C, flags) && (pairs & 7) == 0 && (C != 4 || (wide & 15) == 0)) {
     using Kernel = void (*)(TexArgs);
-    const Kernel kernels[4] = {texture_bwd32_kernel<1>, texture_bwd32_kernel<2>,
-                               texture_bwd32_kernel<3>, texture_bwd32_kernel<4>};
-    kernels[C - 1]<<<unsigned((n + 256 * kPoints - 1) / (256 * kPoints)), 256, 0, stream>>>(a);
+    const Kernel kernels[2][4] = {{texture_bwd32_kernel<1, 1>, texture_bwd32_kernel<2, 1>,
+                                   texture_bwd32_kernel<3, 1>, texture_bwd32_kernel<4, 1>},
+                                  {texture_bwd32_kernel<1, 2>, texture_bwd32_kernel<2, 2>,
+                                   texture_bwd32_kernel<3, 2>, texture_bwd32_kernel<4, 2>}};
+    const int points = points_a_thread(n);
+    kernels[points - 1][C - 1]<<<unsigned((n + 256 * points - 1) / (256 * points)), 256, 0,
+                                 stream>>>(a);
   } else {
     texture_bwd_kernel<<<grid, 256, 0, stream>>>(a);
   }

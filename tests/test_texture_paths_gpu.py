@@ -44,6 +44,33 @@ def test_texture_dispatch(channels, points, offset, device):
     assert (x.cpu().double() - y).abs().max() <= 1e-4 * y.abs().max()
 
 
+# One point a thread up to 466,944 points, two above: both sides of the line, and
+# counts that leave a block one point.
+@pytest.mark.parametrize("points", [466_943, 466_944, 466_945, 467_457, 467_458])
+@pytest.mark.parametrize("channels", [1, 2, 3, 4])
+def test_points_a_thread(points, channels, device):
+  rng = np.random.default_rng(points)
+  tex = rng.uniform(-1, 1, (6, 9, channels)).astype(np.float32)
+  uv = rng.uniform(-0.2, 1.2, (points, 2)).astype(np.float32)
+  g = rng.standard_normal((points, channels)).astype(np.float32)
+  du, dt = _at_offset(uv, 0, device).requires_grad_(), _at_offset(tex, 0, device).requires_grad_()
+  out = shaders.texture_map(du, dt)
+  np.testing.assert_array_equal(out.detach().cpu().numpy(), texture.texture_map(uv, tex))
+  got = torch.autograd.grad(out, (du, dt), _at_offset(g, 0, device))
+  tu = torch.tensor(uv, dtype=torch.float64, requires_grad=True)
+  tt = torch.tensor(tex, dtype=torch.float64, requires_grad=True)
+  want = torch.autograd.grad(texture.texture_map_t(tu, tt), (tu, tt),
+                             torch.tensor(g, dtype=torch.float64))
+  # A coordinate's gradient sums channels x 2 rounded products, as above, but for
+  # the points whose float32 location falls on the other side of a texel's center
+  # (2^-21 of a texel on either axis: some 1e-6 of them). A texel sums up to 4 x
+  # 467k / 54 products of either sign, each within 2^-24 of its magnitude: below
+  # 1e-3 of the largest sum.
+  far = (got[0].cpu().double() - want[0]).abs().max(1).values > 1e-4 * want[0].abs().max()
+  assert far.double().mean() <= 3e-5
+  assert (got[1].cpu().double() - want[1]).abs().max() <= 1e-3 * want[1].abs().max()
+
+
 # float32 rounds sides above 2^24 to even numbers: 2^24 + 3 becomes 2^24 + 4, one
 # past the last padded texel. Coordinates at and beyond the far edge are the last
 # texel and its gradient, those at the near edge the first.
