@@ -211,7 +211,7 @@ class ClockSampler:
     try:
       self.proc = subprocess.Popen(
           ["nvidia-smi", "-i", str(self.gpu), "--query-gpu=" + self.Q,
-           "--format=csv,noheader,nounits", "-lms", "200"],
+           "--format=csv,noheader,nounits", "-lms", "50"],
           stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
       self.thread = threading.Thread(target=self._read, daemon=True)
       self.thread.start()

@@ -1110,30 +1110,28 @@ bool check_config(const dr_raster_config* cfg, int& L, int& TW, int& TH, int& la
 // triangles tell little else: a dense mesh of small triangles and a scene of
 // wide ones, which every tile of the image looks at, count alike.
 //
-// Up to 512 tiles most of the resident blocks (eight on each SM) are idle, and where each tile
-// has work enough smaller ones spread it. Setup to fine kernel, of the time with
-// 16x16 tiles (16 to 2000 triangles a tile, 1 to 8 layers): 0.30 to 1.01 with
-// 8x8 up to 256 tiles, 0.61 to 1.04 with 16x8 up to 512. Below 16 triangles a
-// tile or 4096 in all the launches are what takes the time (up to 1.36 with
-// 8x8). From 600 tiles on both gain on closed meshes (768x768, 100k triangles:
-// 61 us with 16x8, 83) and lose elsewhere: 8x8 up to 1.29 at 4 x 256x256, 16x8
-// up to 1.13 there, and 1.39 on 80k triangles 180 pixels wide at 1024x1024. The
-// threshold of the large list stays the same number of tiles: a fourfold one
-// gained up to a third on triangles of 32 to 64 pixels, for four times the
-// bins' memory.
+// Up to 512 tiles most of the resident blocks (eight on each SM) are idle, and
+// where each tile has work enough smaller ones spread it. Setup to fine kernel,
+// of the time with 16x16 tiles (16 to 2000 triangles a tile, 1 to 8 layers): 0.30
+// to 1.02 with 8x8 up to 256 tiles, 0.61 to 1.04 with 16x8 up to 512. Below 16
+// triangles a tile or 4096 in all the launches are what takes the time (up to
+// 1.36 with 8x8). Above, both gain on closed meshes (100k-triangle sphere at
+// 1283x717, one layer: fine kernel 32 us with 16x8, 49) and lose elsewhere: 8x8 up
+// to 1.24 at 4 x 256x256, 16x8 up to 1.11 there, and 1.35 on 80k triangles 110
+// pixels wide at 1024x1024. The threshold of the large list stays the same number
+// of tiles: a fourfold one gained up to a third on triangles of 32 to 64 pixels,
+// for four times the bins' memory.
 //
 // Many tiles with few triangles each are bound by the cost per tile: the
 // 64-mesh ragged batch (111k tiles) takes 1002 us with 32x16, 1165 with 16x16,
-// 2048x2048 images of triangles 11 to 220 pixels wide 0.50 to 1.03 of 16x16's
-// time, smaller images up to 1.07. With more than 24 triangles a tile 32x16 is
-// no better (terrain 789, 761). An image whose tiles hold more than a 912th of
-// all the triangles each (about a block's share) then sets the time: one with
-// 1531 a tile among 979k took 805 us with 32x16, 514 with 16x16. Above four
-// layers the keys of a 32x16 tile cost more blocks per SM than it gains (eight:
-// 744, 612 on a sphere). It loses too where hundreds of triangles 600 pixels
-// wide lie over each other (up to 1.18 at 2048x2048). 32x8 for rows that do not
-// start on 32 bytes gained 3 to 8% on small triangles and lost up to 28% on
-// wider ones.
+// 2048x2048 images of triangles 11 to 600 pixels wide 0.44 to 1.04 of 16x16's
+// time, smaller images up to 1.09 (the widest triangles). With more than 24
+// triangles a tile 32x16 is no better (terrain 789, 761). An image whose tiles
+// hold more than a 912th of all the triangles each (about a block's share) then
+// sets the time: one with 1531 a tile among 979k took 805 us with 32x16, 514 with
+// 16x16. Above four layers the keys of a 32x16 tile cost more blocks per SM than
+// it gains (eight: 744, 612 on a sphere). 32x8 for rows that do not start on 32
+// bytes gained up to 17% on small triangles and lost up to 18% on wider ones.
 void default_tile(const Batch& b, int L, int& TW, int& TH) {
   const int64_t tiles = b.tile_start[b.n], tris = b.tri_start[b.n];
   TW = TH = kDefaultTile;
