@@ -445,9 +445,9 @@ struct FineSmem {
 // A row pushes up to kPush candidates at a time; fewer than 32 are carried
 // from one push to the next.
 constexpr int kPush = 8, kQueue = 32 * kPush + 32;
-// Between chunks the queues hold gather_large's list.
+// Between chunks the queues hold gather_inline's list.
 static_assert(kThreads / 32 * kQueue * sizeof(unsigned short) >= kThreads * sizeof(int),
-              "gather_large's list");
+              "gather_inline's list");
 
 // Triangles a chunk holds. Up to 768 keys (16x16 pixels of three layers) eight
 // blocks of 128 fit an SM's shared memory, as the registers allow, and every
@@ -692,9 +692,9 @@ __device__ __forceinline__ void fill_background(const RasterArgs& a, const TileB
 // integers. scan: the first triangle of the next group, and how many of that
 // group's hits an earlier chunk took.
 template <int kChunk>
-__device__ __forceinline__ int gather_large(const int32_t* large, int nlarge, const uint2* boxes,
-                                            const int32_t* rest, int nrest, int4 tile, int* list,
-                                            int* s_warp, int2* scan) {
+__device__ __forceinline__ int gather_inline(const int32_t* large, int nlarge, const uint2* boxes,
+                                             const int32_t* rest, int nrest, int4 tile, int* list,
+                                             int* s_warp, int2* scan) {
   const int tid = threadIdx.x;
   int next = scan->x, skip = scan->y;
   int have = max(0, nrest);
@@ -733,6 +733,30 @@ __device__ __forceinline__ int gather_large(const int32_t* large, int nlarge, co
   if (tid == 0) *scan = make_int2(next, skip);
   __syncthreads();
   return tid < have ? list[tid] : -1;
+}
+
+// Inline where the layer count is fixed and the sample outputs are fused; the
+// other instantiations spill 92 bytes with it inline (sphere, 8 x 1024^2: 222,
+// 296 and 406 us at one, two and four layers) and 20 with a call (216, 282, 390),
+// where a call costs the first kind 1 to 3%.
+template <int kChunk>
+__device__ __noinline__ int gather_call(const int32_t* large, int nlarge, const uint2* boxes,
+                                        const int32_t* rest, int nrest, uint32_t x, uint32_t y,
+                                        int* list, int* s_warp, int2* scan) {
+  const int4 tile = make_int4(int(x & 0xffffu), int(x >> 16), int(y & 0xffffu), int(y >> 16));
+  return gather_inline<kChunk>(large, nlarge, boxes, rest, nrest, tile, list, s_warp, scan);
+}
+
+template <int kChunk, bool kInline>
+__device__ __forceinline__ int gather_large(const int32_t* large, int nlarge, const uint2* boxes,
+                                            const int32_t* rest, int nrest, int4 tile, int* list,
+                                            int* s_warp, int2* scan) {
+  if constexpr (kInline)
+    return gather_inline<kChunk>(large, nlarge, boxes, rest, nrest, tile, list, s_warp, scan);
+  else
+    return gather_call<kChunk>(large, nlarge, boxes, rest, nrest,
+                               uint32_t(tile.x) | uint32_t(tile.y) << 16,
+                               uint32_t(tile.z) | uint32_t(tile.w) << 16, list, s_warp, scan);
 }
 
 // Persistent fine rasterizer. Each block takes (image, tile) items from a
@@ -821,9 +845,9 @@ __global__ void __launch_bounds__(kThreads, 8) fine_raster_kernel(RasterArgs a, 
       const int i = c0 + threadIdx.x;
       int cnt = 0, g = -1, cx0 = 0, cy0 = 0, cw = 1;
       if (nlarge > kChunk && c0 + kChunk > nbin) {
-        g = gather_large<kChunk>(a.large_list + tri0, nlarge, a.box, a.bins + bin0 + c0, nbin - c0,
-                                 make_int4(x0, x0 + tw, y0, y0 + th),
-                                 reinterpret_cast<int*>(s.queue), s_warp, &s_scan);
+        g = gather_large<kChunk, (kFused && LT > 0)>(
+            a.large_list + tri0, nlarge, a.box, a.bins + bin0 + c0, nbin - c0,
+            make_int4(x0, x0 + tw, y0, y0 + th), reinterpret_cast<int*>(s.queue), s_warp, &s_scan);
         if (s_scan.x >= nlarge) nsrc = 0;  // the last chunk
       } else if ((kChunk == kThreads || threadIdx.x < kChunk) && i < nsrc) {
         g = i < nbin ? a.bins[bin0 + i] : a.large_list[tri0 + (i - nbin)];
