@@ -1134,10 +1134,10 @@ bool check_config(const dr_raster_config* cfg, int& L, int& TW, int& TH, int& la
 // triangles tell little else: a dense mesh of small triangles and a scene of
 // wide ones, which every tile of the image looks at, count alike.
 //
-// Up to 512 tiles most of the resident blocks (eight on each SM) are idle, and
+// Up to 840 tiles many of the resident blocks (eight on each SM) are idle, and
 // where each tile has work enough smaller ones spread it. Setup to fine kernel,
 // of the time with 16x16 tiles (16 to 2000 triangles a tile, 1 to 8 layers): 0.30
-// to 1.02 with 8x8 up to 256 tiles, 0.61 to 1.04 with 16x8 up to 512. Below 16
+// to 1.02 with 8x8 up to 256 tiles, 0.58 to 1.04 with 16x8 up to 840. Below 16
 // triangles a tile or 4096 in all the launches are what takes the time (up to
 // 1.36 with 8x8). Above, both gain on closed meshes (100k-triangle sphere at
 // 1283x717, one layer: fine kernel 32 us with 16x8, 49) and lose elsewhere: 8x8 up
@@ -1159,7 +1159,7 @@ bool check_config(const dr_raster_config* cfg, int& L, int& TW, int& TH, int& la
 void default_tile(const Batch& b, int L, int& TW, int& TH) {
   const int64_t tiles = b.tile_start[b.n], tris = b.tri_start[b.n];
   TW = TH = kDefaultTile;
-  if (tiles <= 512 && tris >= std::max(int64_t(4096), 16 * tiles)) {
+  if (tiles <= 840 && tris >= std::max(int64_t(4096), 16 * tiles)) {
     TW = tiles <= 256 ? 8 : 16;
     TH = 8;
   } else if (tiles >= 16384 && L <= 4 && tris <= 24 * tiles) {

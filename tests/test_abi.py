@@ -96,12 +96,13 @@ def test_bins_fit_32_bits(tris, w, h):
 
 
 # A smaller default tile shows in the workspace by its tiles' counts (16 bytes
-# each) alone: the triangles' share does not grow with it. It is taken up to 512
+# each) alone: the triangles' share does not grow with it. It is taken up to 840
 # 16x16 tiles with 16 triangles each and 4096 in all, where it never loses.
 @pytest.mark.parametrize("w,h,tris,layers,smaller", [
     (64, 64, 4095, 3, 1), (64, 64, 4096, 3, 4), (256, 256, 4096, 3, 4), (256, 256, 4095, 3, 1),
     (256, 256, 1_000_000, 3, 4), (272, 256, 20_000, 3, 2), (512, 256, 8192, 3, 2),
-    (512, 256, 8191, 3, 1), (512, 256, 40_000_000, 3, 2), (528, 256, 100_000, 3, 1),
+    (512, 256, 8191, 3, 1), (512, 256, 40_000_000, 3, 2), (528, 256, 100_000, 3, 2),
+    (480, 448, 13_440, 3, 2), (480, 448, 13_439, 3, 1), (464, 465, 100_000, 3, 1),
     (512, 512, 20_000, 3, 1), (768, 768, 100_000, 3, 1), (1024, 1024, 80_000, 3, 1),
     (1283, 717, 100_000, 1, 1), (2047, 2048, 1_000_000, 3, 1), (2047, 2048, 1000, 5, 1)])
 def test_default_tile_and_its_workspace(w, h, tris, layers, smaller):
